@@ -2,11 +2,11 @@
 // the model is stored: [out_features, in_features]; the reference's GEMM wrapper has the same
 // contract, src/model/llama.cpp:45-52).
 //
-// * float x float -> float with float FMAs only: the true 32-bit path.  No tensor cores, no
-//   reduced-precision mode.  Every output element is accumulated over k in ascending order by
+// * bfloat16 operands with float accumulation: the plain twin that the fast bfloat16 kernels are checked
+//   against; Y may be float or bfloat16.  Every output element is accumulated over k in ascending order by
 //   one thread, so a row's result does not depend on how many other rows are in the batch.
-// * the same kernel instantiated for bfloat16 operands (float accumulation) is the plain twin
-//   that the fast bfloat16 kernels are checked against; Y may be float or bfloat16.
+// * batches of small products (one per head, say) of either type.
+// Single products of float operands (the true 32-bit path) are gemm_f32.cu.
 #include "common.cuh"
 
 namespace kvcm {
@@ -115,10 +115,6 @@ int launch_gemm_plain(const void* X, const void* W, void* Y, int M, int N, int K
 
 using namespace kvcm;
 
-KVCM_API int kvcm_gemm_plain_f32(const void* X, const void* W, void* Y, int M, int N, int K, int ldx,
-                                 int ldw, int ldy, void* stream) {
-  return launch_gemm_plain<float, float>(X, W, Y, M, N, K, ldx, ldw, ldy, (cudaStream_t)stream);
-}
 KVCM_API int kvcm_gemm_plain_bf16(const void* X, const void* W, void* Y, int M, int N, int K, int ldx,
                                   int ldw, int ldy, void* stream) {
   return launch_gemm_plain<bf16, bf16>(X, W, Y, M, N, K, ldx, ldw, ldy, (cudaStream_t)stream);

@@ -34,7 +34,7 @@ int kvcm_rope_cache_f32(void*, int, const int*, const float*, int, int, const in
 int kvcm_rope_cache_bf16(void*, int, const int*, const float*, int, int, const int*, void*, void*, int, int, int, int, int, int, void*);
 int kvcm_silu_mul_f32(const void*, void*, int, int, void*);
 int kvcm_silu_mul_bf16(const void*, void*, int, int, void*);
-int kvcm_gemm_plain_f32(const void*, const void*, void*, int, int, int, int, int, int, void*);
+int kvcm_gemm_f32(const void*, const void*, void*, int, int, int, int, int, int, int, void*);
 int kvcm_attention_plain_f32(const void*, int, void*, int, const void*, const void*, const int*, int, const int*, const int*,
                              int, int, int, int, int, float, int, float, const float*, void*);
 int kvcm_attention_plain_bf16(const void*, int, void*, int, const void*, const void*, const int*, int, const int*, const int*,
@@ -121,7 +121,7 @@ int library_gemm(const KvcmForwardArgs& a, const void* x, const void* w, void* y
 int product(const KvcmForwardArgs& a, const void* x, const void* w, void* y, int M, int N, int K, bool out_f32,
             cudaStream_t s) {
   if (M == 0) return 0;
-  if (a.f32) return kvcm_gemm_plain_f32(x, w, y, M, N, K, K, K, N, s);
+  if (a.f32) return kvcm_gemm_f32(x, w, y, M, N, K, K, K, N, 1, s);
   if ((M <= 8 || (long long)N * K * 2 <= kStreamMaxBytes) && kvcm_gemm_stream_supports(M, N, K))
     return kvcm_gemm_stream_bf16(x, w, y, M, N, K, K, K, N, out_f32 ? 1 : 0, a.sm_count, s);
   return library_gemm(a, x, w, y, M, N, K, out_f32, s);
@@ -300,7 +300,7 @@ KVCM_API int kvcm_forward(const KvcmForwardArgs* ap, int* launches, void* stream
   if (a.num_logits > 0) {
     KVCM_TRY(rmsnorm(a.x, pending, a.final_norm, 0, a.h_last, a.logit_rows, a.num_logits, H, a.final_eps, s)); ++n;
     if (a.f32) {
-      KVCM_TRY(kvcm_gemm_plain_f32(a.h_last, a.lm_head, a.logits, a.num_logits, a.V, H, H, H, a.V, s));
+      KVCM_TRY(kvcm_gemm_f32(a.h_last, a.lm_head, a.logits, a.num_logits, a.V, H, H, H, a.V, 1, s));
     } else {
       KVCM_TRY(product(a, a.h_last, a.lm_head, a.logits, a.num_logits, a.V, H, true, s));
     }

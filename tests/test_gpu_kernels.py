@@ -155,6 +155,22 @@ def test_plain_gemm_rows_do_not_depend_on_the_batch():
     assert torch.equal(full[20:21], one)
 
 
+@pytest.mark.parametrize("M,N,Kd,ld", [(1, 5, 1, 0), (4, 64, 255, 0), (5, 65, 256, 0), (16, 130, 1021, 3), (17, 127, 1024, 4),
+                                       (96, 200, 2056, 0), (97, 129, 516, 0), (200, 77, 2045, 0), (3, 70, 5632, 0)])
+def test_float32_product_at_the_edges_of_its_tiles(M, N, Kd, ld):
+    """Every tile form, segment count and copy width.  A chain of a segment's even or odd k's has at most
+    ceil(K / 2S) + 4 FMAs and the sums join in at most 8 additions, so |error| <= (ceil(K / 2S) + 12) * 2^-24 * sum |x w|;
+    a row alone gives the bits it gives beside others."""
+    x, w = torch.randn(M, Kd + ld, device=DEV)[:, :Kd], torch.randn(N, Kd, device=DEV)
+    y, one = torch.full((M, N), float("nan"), device=DEV), torch.empty(1, N, device=DEV)
+    K().gemm_plain(x, w, y)
+    S = 8 if Kd >= 1024 else 4 if Kd >= 512 else 2 if Kd >= 256 else 1
+    bound = (Kd // (2 * S) + 13) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)
+    assert bool(((y.double() - x.double() @ w.double().T).abs() <= bound).all())
+    K().gemm_plain(x[M - 1:], w, one)
+    assert torch.equal(one, y[M - 1:])
+
+
 @pytest.mark.parametrize("M,N,Kd", [(1, 2048, 2048), (8, 2560, 2048), (3, 100, 176), (16, 37, 2048), (8, 37, 5632),
                                     (9, 515, 96), (8, 32003, 256), (5, 16, 8), (8, 11264, 2048),
                                     (7, 4096, 1032), (2, 33, 520),
