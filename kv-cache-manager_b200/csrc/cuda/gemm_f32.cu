@@ -14,10 +14,11 @@
 // * The even and the odd chain are the halves of one packed FMA (fma.rn.f32x2): a 16-byte read is its operand
 //   pair as it lies, and the issue slots needed are halved.
 // * The weights of the first stages are requested before the dependency wait where the caller vouches for them.
-// Measured on B200 at the 1.1B shape, W [11264, 2048]: 2 rows 35 us (2.6 TB/s of weights), 64 rows 109 us (27
-// TFLOP/s), 600 rows 866 us (32 TFLOP/s).  Before, one block per 64 x 64 outputs walked the whole of K, whatever the
-// number of rows: 370 to 1,200 us a product of this model at 2 to 130 rows (two prompts of 64 tokens, 8 steps and
-// their score: 466 ms, now 38 ms).  Error against 64 bits over that whole run: 2.6e-6 before, 7.3e-7 now.
+// * A thread's addresses are formed once: a few warps an SM run the copies, and their instructions were the bound.
+// Measured on B200 at the 1.1B shape, W [11264, 2048]: 2 rows 21 us (4.3 TB/s of weights; 35 us with the addresses formed
+// piece by piece), 600 rows 688 us (40 TFLOP/s).  Before, one block per 64 x 64 outputs walked the whole of K, whatever the
+// number of rows: 370 to 1,200 us a product of this model at 2 to 130 rows.  Error against 64 bits over a run of two
+// prompts of 64 tokens, 8 steps and their score: 2.6e-6 before, 7.3e-7 now.
 #include <cooperative_groups.h>
 
 #include "common.cuh"
@@ -66,16 +67,33 @@ gemm_f32_kernel(const float* __restrict__ X, const float* __restrict__ W, float*
   const int k0 = min(rank * seg, K), k1 = min(k0 + seg, K);
   const int steps = (k1 - k0 + kF32K - 1) / kF32K;
 
-  const auto load = [&](const float* __restrict__ P, int ld, int rows, int first, int limit, int step, float* dst) {
-    const int kb = k0 + step * kF32K;
-    for (int p = tid; p < rows * PIECES; p += C::THREADS) {
-      const int r = p / PIECES, c = (p % PIECES) * PIECE;
-      const bool ok = first + r < limit && kb + c < k1;
-      copy_async<PIECE * 4>(dst + r * kF32Pitch + c, ok ? P + size_t(first + r) * ld + kb + c : P, ok);
+  // This thread's piece of a row of a stage, and every RSTEP-th row from r0 on: addresses are formed once.
+  constexpr int RSTEP = C::THREADS / PIECES;
+  static_assert(C::THREADS % PIECES == 0 && BN % RSTEP == 0 && (BM % RSTEP == 0 || BM < RSTEP), "copies tile the stage");
+  const int r0 = tid / PIECES, c0 = (tid % PIECES) * PIECE;
+  const float* const w_from = W + size_t(n0 + r0) * ldw + k0 + c0;
+  const float* const x_from = X + size_t(m0 + r0) * ldx + k0 + c0;
+  const size_t w_rstep = size_t(RSTEP) * ldw, x_rstep = size_t(RSTEP) * ldx;
+  const int w_live = N - n0 - r0, x_live = M - m0 - r0;           // rows i * RSTEP below these exist
+  const auto load_w = [&](int step) {
+    const bool in = k0 + step * kF32K + c0 < k1;
+    float* dst = f32_smem + (step % STAGES) * STAGE + (BM + r0) * kF32Pitch + c0;
+#pragma unroll
+    for (int i = 0; i < BN / RSTEP; ++i) {
+      const bool ok = in && i * RSTEP < w_live;
+      copy_async<PIECE * 4>(dst + i * RSTEP * kF32Pitch, ok ? w_from + i * w_rstep + step * kF32K : W, ok);
     }
   };
-  const auto load_w = [&](int step) { load(W, ldw, BN, n0, N, step, f32_smem + (step % STAGES) * STAGE + BM * kF32Pitch); };
-  const auto load_x = [&](int step) { load(X, ldx, BM, m0, M, step, f32_smem + (step % STAGES) * STAGE); };
+  const auto load_x = [&](int step) {
+    const bool in = k0 + step * kF32K + c0 < k1;
+    float* dst = f32_smem + (step % STAGES) * STAGE + r0 * kF32Pitch + c0;
+    if (BM % RSTEP != 0 && r0 >= BM) return;
+#pragma unroll
+    for (int i = 0; i < (BM + RSTEP - 1) / RSTEP; ++i) {
+      const bool ok = in && i * RSTEP < x_live;
+      copy_async<PIECE * 4>(dst + i * RSTEP * kF32Pitch, ok ? x_from + i * x_rstep + step * kF32K : X, ok);
+    }
+  };
 
   pdl_launch_dependents();
   if (!weights_ready) pdl_wait();
@@ -169,18 +187,24 @@ static int launch_tile(const float* X, const float* W, float* Y, int M, int N, i
                             ldx, ldw, ldy, S, seg, int(mtiles), weights_ready);
 }
 
+// Which tile.  Up to 16 rows read the weights once: a narrow N leaves few blocks, which then take small tiles and deep
+// rings; a wide N makes more blocks than run at once, which then take little shared memory each.  Beyond, the smallest
+// padding of the rows; tiles of 48 rows run at 0.85 of the rate of tiles of 64.  Measured in us on B200 (W [11264, 2048] | [2048,
+// 5632]): 2 rows 21 | 12.5 (the other form 28 | 22), 8 rows 27.5 | 21.7 (30 | 30), 16 rows 32 | 24 (42 | 34), 32 rows 52 | 45, 64
+// rows 87 | 48 (in tiles of 32: 90; in tiles of 64: 76), 72 rows 124 | 64 (in tiles of 64: 160 | 77), 600 rows 688 | 358.
 template <bool VEC>
 static int launch(const float* X, const float* W, float* Y, int M, int N, int K, int ldx, int ldw, int ldy, int weights_ready,
                   cudaStream_t s) {
-  using Few = F32Tile<4, 64, 2, 1, 32, 6>;
-  using Some = F32Tile<16, 64, 4, 2, 8, 5>;
-  using Rows32 = F32Tile<32, 128, 8, 4, 8, 4>;
-  using Rows64 = F32Tile<64, 128, 8, 8, 8, 3>;
-  // the smallest tile that holds the rows; beyond 16, tiles of 32 while they pad less than tiles of 64 would
-  if (M <= Few::BM) return launch_tile<Few, VEC>(X, W, Y, M, N, K, ldx, ldw, ldy, weights_ready, s);
-  if (M <= Some::BM) return launch_tile<Some, VEC>(X, W, Y, M, N, K, ldx, ldw, ldy, weights_ready, s);
-  if (M <= 96) return launch_tile<Rows32, VEC>(X, W, Y, M, N, K, ldx, ldw, ldy, weights_ready, s);
-  return launch_tile<Rows64, VEC>(X, W, Y, M, N, K, ldx, ldw, ldy, weights_ready, s);
+#define KVCM_F32_TILE(...) return launch_tile<F32Tile<__VA_ARGS__>, VEC>(X, W, Y, M, N, K, ldx, ldw, ldy, weights_ready, s)
+  const bool narrow = N <= 4096;
+  if (M <= 4) { if (narrow) KVCM_F32_TILE(4, 32, 2, 1, 32, 8); else KVCM_F32_TILE(4, 64, 2, 1, 32, 3); }
+  if (M <= 8) { if (narrow) KVCM_F32_TILE(8, 32, 4, 1, 16, 4); else KVCM_F32_TILE(8, 64, 4, 1, 16, 3); }
+  if (M <= 16) { if (narrow) KVCM_F32_TILE(16, 64, 4, 2, 8, 5); else KVCM_F32_TILE(16, 64, 8, 2, 16, 3); }
+  if (M <= 32 || (M > 48 && M <= 64 && narrow)) KVCM_F32_TILE(32, 64, 8, 4, 16, 4);
+  if (M <= 48) KVCM_F32_TILE(48, 64, 6, 4, 16, 4);
+  if ((M + 47) / 48 * 55 < (M + 63) / 64 * 64) KVCM_F32_TILE(48, 64, 6, 8, 8, 3);
+  KVCM_F32_TILE(64, 64, 8, 8, 8, 3);
+#undef KVCM_F32_TILE
 }
 
 }  // namespace kvcm
