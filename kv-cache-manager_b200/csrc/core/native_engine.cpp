@@ -71,9 +71,8 @@ NativeEngine::NativeEngine(KVManager& kv, Scheduler& sched, NativeModel model, N
   }
   d_ints_ = static_cast<int32_t*>(device(size_t(capacity_) * 4));
   d_packed_ = static_cast<int32_t*>(device(size_t(2 + max_logits_) * 4));
-  sampling_bytes_ = size_t(max_logits_) * (4 + 4 + 8 + 8);
-  h_sampling_ = static_cast<unsigned char*>(host(sampling_bytes_));
-  d_sampling_ = static_cast<unsigned char*>(device(sampling_bytes_));
+  for (int i = 0; i < 2; ++i) h_sampling_[i] = static_cast<unsigned char*>(host(24 * sampling_rows(max_logits_)));
+  d_sampling_ = static_cast<unsigned char*>(device(24 * sampling_rows(max_logits_)));
   x_ = device(T * H * 4);
   h_ = device(T * H * esz);
   proj_ = device(T * H * esz);
@@ -84,7 +83,7 @@ NativeEngine::NativeEngine(KVManager& kv, Scheduler& sched, NativeModel model, N
   h_last_ = device(size_t(max_logits_) * H * esz);
   logits_ = device(size_t(max_logits_) * model_.V * 4);
   if (cfg_.attn_scratch_floats > 0) attn_scratch_ = device(size_t(cfg_.attn_scratch_floats) * 4);
-  if (cfg_.fuse_norms && !model_.f32) norm_partials_ = device(size_t((model_.H + 15) / 16 * 16) * 4);
+  if (cfg_.fuse_norms && !model_.f32) norm_partials_ = device(size_t((model_.H + 127) / 128 * 128) * 4);
   if (!model_.f32) rope_table_ = device(size_t(cfg_.max_rows) * model_.hd * 4);
   if (!model_.f32 && cfg_.lib_workspace_bytes > 0) lib_ws_ = device(size_t(cfg_.lib_workspace_bytes));
 }
@@ -100,11 +99,11 @@ NativeEngine::~NativeEngine() {
   for (int i = 0; i < 2; ++i) {
     if (h_ints_[i]) dev_.host_free(h_ints_[i]);
     if (h_packed_[i]) dev_.host_free(h_packed_[i]);
+    if (h_sampling_[i]) dev_.host_free(h_sampling_[i]);
     if (ev0_[i]) dev_.event_destroy(ev0_[i]);
     if (ev1_[i]) dev_.event_destroy(ev1_[i]);
     if (done_[i]) dev_.event_destroy(done_[i]);
   }
-  if (h_sampling_) dev_.host_free(h_sampling_);
   if (stream_) dev_.stream_destroy(stream_);
 }
 
@@ -142,7 +141,7 @@ void NativeEngine::fill_args(KvcmForwardArgs& a, const BatchLayout& L, const int
   a.rope_table = static_cast<float*>(rope_table_);
   a.rope_table_floats = rope_table_ ? (long long)cfg_.max_rows * model_.hd : 0;
   a.norm_partials = static_cast<float*>(norm_partials_);
-  a.norm_partials_floats = norm_partials_ ? (model_.H + 15) / 16 * 16 : 0;
+  a.norm_partials_floats = norm_partials_ ? (model_.H + 127) / 128 * 128 : 0;
   a.lib_workspace = lib_ws_;
   a.lib_workspace_bytes = lib_ws_ ? cfg_.lib_workspace_bytes : 0;
   a.num_layers = static_cast<int>(model_.layers.size());
@@ -163,12 +162,13 @@ void NativeEngine::fill_args(KvcmForwardArgs& a, const BatchLayout& L, const int
 }
 
 // Per-row sampling parameters of the plan's entries that sample, rows beyond them greedy.
-void NativeEngine::stage_sampling(const std::vector<ScheduledSeq>& plan, int rows) {
-  const size_t R = size_t(max_logits_);
-  float* temps = reinterpret_cast<float*>(h_sampling_);
-  int32_t* pos = reinterpret_cast<int32_t*>(h_sampling_ + 4 * R);
-  uint64_t* seeds = reinterpret_cast<uint64_t*>(h_sampling_ + 8 * R);
-  int64_t* ids = reinterpret_cast<int64_t*>(h_sampling_ + 16 * R);
+size_t NativeEngine::pack_sampling(const std::vector<ScheduledSeq>& plan, int rows, int parity) {
+  const size_t R = sampling_rows(rows);
+  unsigned char* to = h_sampling_[parity];
+  float* temps = reinterpret_cast<float*>(to);
+  int32_t* pos = reinterpret_cast<int32_t*>(to + 4 * R);
+  uint64_t* seeds = reinterpret_cast<uint64_t*>(to + 8 * R);
+  int64_t* ids = reinterpret_cast<int64_t*>(to + 16 * R);
   int n = 0;
   for (const ScheduledSeq& p : plan) {
     if (!p.wants_logits) continue;
@@ -178,27 +178,39 @@ void NativeEngine::stage_sampling(const std::vector<ScheduledSeq>& plan, int row
     ids[n] = p.seq->id;
     ++n;
   }
-  for (; n < rows; ++n) { temps[n] = 0.f; pos[n] = 0; seeds[n] = 0; ids[n] = 0; }
-  check(dev_.copy_to_device(d_sampling_, h_sampling_, sampling_bytes_, stream_), "copying the sampling parameters");
+  for (; n < static_cast<int>(R); ++n) { temps[n] = 0.f; pos[n] = 0; seeds[n] = 0; ids[n] = 0; }
+  return 24 * R;
+}
+
+size_t NativeEngine::stage_sampling(const std::vector<ScheduledSeq>& plan, int rows, int parity) {
+  const size_t bytes = pack_sampling(plan, rows, parity);
+  check(dev_.copy_to_device(d_sampling_, h_sampling_[parity], bytes, stream_), "copying the sampling parameters");
+  return bytes;
 }
 
 int NativeEngine::run_device(const KvcmForwardArgs& a, int logit_rows, bool tempered, const int32_t* fetch_from,
-                             int32_t* fetch_to, long long fetch_ints, int32_t* mirror) {
+                             int32_t* fetch_to, long long fetch_ints, int32_t* mirror,
+                             const unsigned char* fetch_sampling) {
   int launches = 0, extra = 0;
+  const size_t R = sampling_rows(logit_rows);
   if (fetch_from != nullptr) {
     check(dev_.fetch_ints(fetch_from, fetch_to, fetch_ints, stream_), "fetching the batch");
     extra = 1;
   }
+  if (fetch_sampling != nullptr) {
+    check(dev_.fetch_ints(reinterpret_cast<const int*>(fetch_sampling), reinterpret_cast<int*>(d_sampling_), (long long)(6 * R), stream_),
+          "fetching the sampling parameters");
+    ++extra;
+  }
   check(dev_.forward(&a, &launches, stream_), "the forward pass");
   launches += extra;
   if (logit_rows > 0) {
-    const size_t R = size_t(max_logits_);
     if (tempered)
       check(dev_.sample(static_cast<const float*>(logits_), reinterpret_cast<const float*>(d_sampling_),
                         reinterpret_cast<const unsigned long long*>(d_sampling_ + 8 * R),
                         reinterpret_cast<const long long*>(d_sampling_ + 16 * R),
                         reinterpret_cast<const int*>(d_sampling_ + 4 * R), d_packed_ + 2, logit_rows, model_.V, d_packed_,
-                        stream_),
+                        mirror, stream_),
             "the sampling kernel");
     else
       check(dev_.argmax(static_cast<const float*>(logits_), d_packed_ + 2, logit_rows, model_.V, d_packed_, mirror,
@@ -243,8 +255,8 @@ NativeEngine::Planned NativeEngine::summarise() {
 
 // Records the forms of a decode shape: token ids from the batch arrays and copies by command (the
 // first step of a run of decode steps), and the chained form of the lookahead, once per pair of
-// pinned buffers: token ids from the sampled tokens of the step before, the batch arrays fetched by a
-// kernel, the tokens written to pinned memory by the sampling kernel.
+// pinned buffers: token ids from the sampled tokens of the step before, the batch arrays (and the sampling
+// parameters) fetched by a kernel, the tokens written to pinned memory by the sampling kernel.
 void NativeEngine::record_shape(Captured& c, const KvcmForwardArgs& args, int b, bool tempered) {
   for (int form = 0; form < 3; ++form) {
     KvcmForwardArgs a = args;
@@ -254,7 +266,8 @@ void NativeEngine::record_shape(Captured& c, const KvcmForwardArgs& args, int b,
     if (rc == 0) {
       try {
         if (form == 0) run_device(a, b, tempered);
-        else run_device(a, b, tempered, h_ints_[form - 1], c.ints, (c.total_ints + 3) / 4 * 4, h_packed_[form - 1]);
+        else run_device(a, b, tempered, h_ints_[form - 1], c.ints, (c.total_ints + 3) / 4 * 4, h_packed_[form - 1],
+                        tempered ? h_sampling_[form - 1] : nullptr);
       } catch (...) {
         void* dead = nullptr;
         dev_.graph_end(stream_, &dead);
@@ -264,7 +277,7 @@ void NativeEngine::record_shape(Captured& c, const KvcmForwardArgs& args, int b,
       rc = dev_.graph_end(stream_, exec);
     }
     check(rc, "recording a CUDA graph");
-    if (tempered || !cfg_.lookahead) break;               // the chained forms serve greedy steps only
+    if (!cfg_.lookahead) break;
   }
 }
 
@@ -278,12 +291,13 @@ NativeStepInfo NativeEngine::run_planned(const Planned& p, double t_start) {
   const int n = p.n, wants = p.wants;
   const bool decode_only = cfg_.graphs && p.singles == n && wants == n;
   KvcmForwardArgs args;
+  size_t sampling_bytes = 0;
   if (decode_only) {
     const int b = std::min(batch_bucket(n), std::max(max_logits_, n));
     const BatchLayout L = builder_.build(entries_, h_ints_[par], capacity_, b, b, b);
     t_built = now();
     const auto key = std::make_tuple(b, ctx_bucket(L.max_decode_ctx), p.tempered > 0 ? 1 : 0);
-    if (p.tempered > 0) stage_sampling(plan, b);
+    if (p.tempered > 0) sampling_bytes = stage_sampling(plan, b, par);
     auto it = graphs_.find(key);
     if (it == graphs_.end()) {
       // Record this shape.  The step at hand runs eagerly first (lazy set-up of kernels and of the
@@ -324,12 +338,12 @@ NativeStepInfo NativeEngine::run_planned(const Planned& p, double t_start) {
       info.launches = c.launches;
       info.graph = true;
     }
-    info.h2d_bytes = L.total_ints * 4 + (p.tempered > 0 ? static_cast<long long>(sampling_bytes_) : 0);
+    info.h2d_bytes = L.total_ints * 4 + static_cast<long long>(sampling_bytes);
   } else {
     const BatchLayout L = builder_.build(entries_, h_ints_[par], capacity_);
     t_built = now();
     check(dev_.copy_to_device(d_ints_, h_ints_[par], size_t(L.total_ints) * 4, stream_), "copying the batch");
-    if (wants > 0 && p.tempered > 0) stage_sampling(plan, wants);
+    if (wants > 0 && p.tempered > 0) sampling_bytes = stage_sampling(plan, wants, par);
     fill_args(args, L, d_ints_, L.max_decode_ctx);
     if (timing_) check(dev_.event_record(ev0_[par], stream_), "recording an event");
     info.launches = run_device(args, wants, p.tempered > 0);
@@ -338,7 +352,7 @@ NativeStepInfo NativeEngine::run_planned(const Planned& p, double t_start) {
       check(dev_.copy_to_host(h_packed_[par], d_packed_, size_t(2 + wants) * 4, stream_), "reading the tokens back");
     t_enqueued = now();
     check(dev_.stream_sync(stream_), "waiting for the step");
-    info.h2d_bytes = L.total_ints * 4 + (wants > 0 && p.tempered > 0 ? static_cast<long long>(sampling_bytes_) : 0);
+    info.h2d_bytes = L.total_ints * 4 + static_cast<long long>(sampling_bytes);
   }
   if (timing_) {
     float ms = 0.f;
@@ -373,7 +387,7 @@ NativeStepInfo NativeEngine::run_planned(const Planned& p, double t_start) {
   return info;
 }
 
-// A greedy decode step of a recorded shape, enqueued and not waited for.  `chained`: the token ids
+// A decode step of a recorded shape, enqueued and not waited for.  `chained`: the token ids
 // are the tokens that the step before it samples (it is still on the device).  False: this step
 // cannot go that way (its shape is not recorded yet, or not in both forms).
 bool NativeEngine::enqueue_decode(const Planned& p, bool chained, double t_start) {
@@ -381,10 +395,12 @@ bool NativeEngine::enqueue_decode(const Planned& p, bool chained, double t_start
   const int b = std::min(batch_bucket(n), std::max(max_logits_, n));
   const int par = int(step_no_ & 1);
   const BatchLayout L = builder_.build(entries_, h_ints_[par], capacity_, b, b, b);
-  auto it = graphs_.find(std::make_tuple(b, ctx_bucket(L.max_decode_ctx), 0));
+  auto it = graphs_.find(std::make_tuple(b, ctx_bucket(L.max_decode_ctx), p.tempered > 0 ? 1 : 0));
   if (it == graphs_.end() || it->second.exec_chained[par] == nullptr || it->second.total_ints != L.total_ints) return false;
   ++step_no_;
   Captured& c = it->second;
+  size_t sampling_bytes = 0;
+  if (p.tempered > 0) sampling_bytes = chained ? pack_sampling(sched_.plan(), b, par) : stage_sampling(sched_.plan(), b, par);
   if (chained) {
     // no copy commands: the recording fetches h_ints_[par] itself and writes its tokens into
     // h_packed_[par], which holds -1 until then
@@ -415,7 +431,7 @@ bool NativeEngine::enqueue_decode(const Planned& p, bool chained, double t_start
   flight_.info.sampled = p.wants;
   flight_.info.launches = c.launches;
   flight_.info.graph = true;
-  flight_.info.h2d_bytes = L.total_ints * 4;
+  flight_.info.h2d_bytes = L.total_ints * 4 + static_cast<long long>(sampling_bytes);
   flight_.info.d2h_bytes = 4ll * (2 + n);
   for (const ScheduledSeq& q : sched_.plan()) {
     flight_.seqs.push_back(q.seq);
@@ -488,11 +504,11 @@ NativeStepInfo NativeEngine::step() {
     planned_ = false;
     if (sched_.plan().empty()) return NativeStepInfo{};
     const Planned p = summarise();
-    const bool greedy_decode = cfg_.graphs && cfg_.lookahead && p.singles == p.n && p.wants == p.n && p.tempered == 0;
-    if (!greedy_decode || !enqueue_decode(p, false, t_start)) return run_planned(p, t_start);
+    const bool decode_only = cfg_.graphs && cfg_.lookahead && p.singles == p.n && p.wants == p.n;
+    if (!decode_only || !enqueue_decode(p, false, t_start)) return run_planned(p, t_start);
     host_.schedule += now() - t_start;
   }
-  // A greedy decode step is on the device.  Put placeholders where its tokens will go, so that the
+  // A decode step is on the device.  Put placeholders where its tokens will go, so that the
   // scheduler can plan the step after it, and enqueue that one behind it if the batch stays as it is.
   InFlight cur = std::move(flight_);
   flight_ = InFlight{};
@@ -509,8 +525,7 @@ NativeStepInfo NativeEngine::step() {
     const std::vector<ScheduledSeq>& plan = sched_.plan();
     same = static_cast<int>(plan.size()) == cur.n && sched_.counters().preemptions == evictions;
     for (int i = 0; same && i < cur.n; ++i)
-      same = plan[i].seq.get() == cur.seqs[i].get() && plan[i].num_tokens == 1 && plan[i].wants_logits &&
-             plan[i].seq->sampling.temperature <= 0.f;
+      same = plan[i].seq.get() == cur.seqs[i].get() && plan[i].num_tokens == 1 && plan[i].wants_logits;
     if (same) {
       const Planned p = summarise();
       const double t_built = now();
@@ -575,8 +590,8 @@ int fake_fetch_ints(const int* src, int* dst, long long ints, void*) {
   return 0;
 }
 int fake_sample(const float* logits, const float*, const unsigned long long*, const long long*, const int*, int* out,
-                int rows, int vocab, int* status, void* s) {
-  return fake_argmax(logits, out, rows, vocab, status, nullptr, s);
+                int rows, int vocab, int* status, int* mirror, void* s) {
+  return fake_argmax(logits, out, rows, vocab, status, mirror, s);
 }
 int fake_copy(void* dst, const void* src, size_t bytes, void*) { std::memcpy(dst, src, bytes); return 0; }
 int fake_stream_create(void** s) { *s = reinterpret_cast<void*>(0x1); return 0; }

@@ -16,8 +16,10 @@
 // device (a second recording of each shape reads its tokens from there).  Everything else a decode
 // step needs (positions, page slots, context lengths, page tables) follows from the lengths alone.
 // The host then waits for step k's tokens only, puts them into the requests, and returns step k.
+// A request that samples with a temperature is no exception: its draw depends on the seed, the request and the
+// position only, which the host knows beforehand; a step's parameters lie in pinned memory beside its batch arrays.
 // So the device never waits for the host between decode steps.  This holds only while the batch
-// stays what it was: all requests decode greedily, none ends, none arrives, no page runs out; the
+// stays what it was: all requests decode, none ends, none arrives, no page runs out; the
 // moment one of these fails the loop waits for the tokens first, as before.  It is switched off where
 // a token's value decides what happens next (an end-of-sequence token) or enters host state at once
 // (page hashes of the prefix cache).
@@ -129,8 +131,13 @@ class NativeEngine {
   void fill_args(KvcmForwardArgs& a, const BatchLayout& L, const int32_t* base, int max_decode_ctx) const;
   // forward + sampling; launches made.  `fetch_from` / `mirror`: the chained form (pinned buffers of one parity).
   int run_device(const KvcmForwardArgs& a, int logit_rows, bool tempered, const int32_t* fetch_from = nullptr,
-                 int32_t* fetch_to = nullptr, long long fetch_ints = 0, int32_t* mirror = nullptr);
-  void stage_sampling(const std::vector<ScheduledSeq>& plan, int rows);
+                 int32_t* fetch_to = nullptr, long long fetch_ints = 0, int32_t* mirror = nullptr,
+                 const unsigned char* fetch_sampling = nullptr);
+  // Packs the sampling parameters of `rows` rows into the pinned buffer of this parity: temperatures | positions | seeds |
+  // ids, each as long as sampling_rows(rows).  Returns their bytes.
+  size_t pack_sampling(const std::vector<ScheduledSeq>& plan, int rows, int parity);
+  size_t stage_sampling(const std::vector<ScheduledSeq>& plan, int rows, int parity);      // ... and copies them
+  static size_t sampling_rows(int rows) { return size_t(rows + 1) / 2 * 2; }                // (24 bytes a row: multiples of 16)
   [[noreturn]] void raise_status(int first, int word);
 
   KVManager& kv_;
@@ -153,9 +160,8 @@ class NativeEngine {
   int32_t* d_ints_ = nullptr;                                 // before it is still being copied
   int32_t* h_packed_[2] = {nullptr, nullptr};                 // [status pair | tokens]
   int32_t* d_packed_ = nullptr;
-  unsigned char* h_sampling_ = nullptr;                       // temps | positions | seeds | ids
+  unsigned char* h_sampling_[2] = {nullptr, nullptr};
   unsigned char* d_sampling_ = nullptr;
-  size_t sampling_bytes_ = 0;
   void *x_ = nullptr, *h_ = nullptr, *qkv_ = nullptr, *attn_ = nullptr, *proj_ = nullptr, *gate_up_ = nullptr,
        *act_ = nullptr, *h_last_ = nullptr, *logits_ = nullptr, *attn_scratch_ = nullptr, *lib_ws_ = nullptr,
        *norm_partials_ = nullptr, *rope_table_ = nullptr;

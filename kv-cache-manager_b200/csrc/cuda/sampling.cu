@@ -55,12 +55,24 @@ __device__ void block_argmax(const float* __restrict__ row, int vocab, float& be
   int bi = 0x7fffffff;
   if ((vocab & 3) == 0 && (reinterpret_cast<uintptr_t>(row) & 15) == 0) {
     // four consecutive logits per load; within a thread indices still ascend
-    for (int i = threadIdx.x * 4; i < vocab; i += blockDim.x * 4) {
-      const float4 v = *reinterpret_cast<const float4*>(row + i);
-      if (v.x > bv) { bv = v.x; bi = i; }
-      if (v.y > bv) { bv = v.y; bi = i + 1; }
-      if (v.z > bv) { bv = v.z; bi = i + 2; }
-      if (v.w > bv) { bv = v.w; bi = i + 3; }
+    // (a block has a row to itself, so its loads' latency is what counts: eight are in flight, and a trip covers 32,768
+    // logits; 32,000 of them one load at a time were eight latencies)
+    constexpr int kAhead = 8;
+    for (int i0 = threadIdx.x * 4; i0 < vocab; i0 += kAhead * blockDim.x * 4) {
+      float4 v[kAhead];
+#pragma unroll
+      for (int k = 0; k < kAhead; ++k) {
+        const int i = i0 + k * blockDim.x * 4;
+        v[k] = i < vocab ? *reinterpret_cast<const float4*>(row + i) : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+      }
+#pragma unroll
+      for (int k = 0; k < kAhead; ++k) {
+        const int i = i0 + k * blockDim.x * 4;
+        if (v[k].x > bv) { bv = v[k].x; bi = i; }
+        if (v[k].y > bv) { bv = v[k].y; bi = i + 1; }
+        if (v[k].z > bv) { bv = v[k].z; bi = i + 2; }
+        if (v[k].w > bv) { bv = v[k].w; bi = i + 3; }
+      }
     }
   } else {
     for (int i = threadIdx.x; i < vocab; i += blockDim.x) {
@@ -118,13 +130,15 @@ __device__ __forceinline__ float sampling_uniform(unsigned long long seed, long 
 __global__ void __launch_bounds__(kSampleThreads)
 sample_kernel(const float* __restrict__ logits, const float* __restrict__ temperature,
               const unsigned long long* __restrict__ seed, const long long* __restrict__ request_id,
-              const int* __restrict__ position, int* __restrict__ out, int vocab, StatusWords sw, int* status) {
-  if (status != nullptr && blockIdx.x == 0 && threadIdx.x == 0) gather_status(sw, status, nullptr);
+              const int* __restrict__ position, int* __restrict__ out, int vocab, StatusWords sw, int* status, int* mirror) {
   __shared__ float sv[32];
   __shared__ int si[32];
-  __shared__ float part[kSampleThreads];
-  __shared__ int chosen_segment;
-  __shared__ float segment_base, target;
+  __shared__ __align__(16) float part[kSampleThreads], upto[kSampleThreads];   // a segment's sum; the sums up to and with it
+  __shared__ int first_past, last_filled;
+  __shared__ float total;
+  pdl_launch_dependents();
+  pdl_wait();
+  if (status != nullptr && blockIdx.x == 0 && threadIdx.x == 0) gather_status(sw, status, mirror);
   const int r = blockIdx.x;
   const float* row = logits + size_t(r) * vocab;
   float best;
@@ -132,7 +146,10 @@ sample_kernel(const float* __restrict__ logits, const float* __restrict__ temper
   block_argmax(row, vocab, best, index, sv, si);
   const float temp = temperature[r];
   if (!(temp > 0.f)) {
-    if (threadIdx.x == 0) out[r] = index;
+    if (threadIdx.x == 0) {
+      out[r] = index;
+      if (mirror != nullptr) *reinterpret_cast<volatile int*>(mirror + 2 + r) = index;
+    }
     return;
   }
   const float inv_t = 1.f / temp;
@@ -142,37 +159,43 @@ sample_kernel(const float* __restrict__ logits, const float* __restrict__ temper
   for (int i = begin; i < end; ++i) s += expf((row[i] - best) * inv_t);
   part[threadIdx.x] = s;
   __syncthreads();
+  // One thread adds the segments up in order and leaves every prefix (a draw must not depend on how the sums are
+  // split); all then look for the segment at once: the first filled one whose prefix lies past the target, or, where
+  // rounding pushed the target past the end, the last filled one.
   if (threadIdx.x == 0) {
-    float total = 0.f;
-    for (int i = 0; i < kSampleThreads; ++i) total += part[i];
-    const float want = sampling_uniform(seed[r], request_id[r], position[r]) * total;
+    first_past = kSampleThreads;
+    last_filled = -1;
+    const int filled = (vocab + seg - 1) / seg;
     float run = 0.f;
-    int pick = -1;
-    for (int i = 0; i < kSampleThreads; ++i) {
-      if (part[i] > 0.f) {
-        pick = i;                                   // last non-empty segment so far: the fallback
-        if (want < run + part[i]) break;
-      }
-      run += part[i];
+    for (int i = 0; i < filled; i += 4) {                    // (part[] is zero beyond the last segment)
+      const float4 t = *reinterpret_cast<const float4*>(part + i);
+      float4 u;
+      u.x = run + t.x; u.y = u.x + t.y; u.z = u.y + t.z; u.w = u.z + t.w;
+      *reinterpret_cast<float4*>(upto + i) = u;
+      run = u.w;
     }
-    if (pick >= 0 && !(want < run + part[pick])) {  // rounding pushed `want` past the end
-      run = 0.f;
-      for (int i = 0; i < pick; ++i) run += part[i];
-    }
-    chosen_segment = pick;
-    segment_base = run;
-    target = want;
+    total = run;
   }
   __syncthreads();
-  if (threadIdx.x == chosen_segment) {
-    float run = segment_base;
+  const float target = sampling_uniform(seed[r], request_id[r], position[r]) * total;
+  if (s > 0.f) {
+    if (target < upto[threadIdx.x]) atomicMin(&first_past, int(threadIdx.x));
+    atomicMax(&last_filled, int(threadIdx.x));
+  }
+  __syncthreads();
+  const int chosen = first_past < kSampleThreads ? first_past : last_filled;
+  if (threadIdx.x == chosen) {
+    float run = chosen > 0 ? upto[chosen - 1] : 0.f;
     int pick = end - 1;
     for (int i = begin; i < end; ++i) {
       run += expf((row[i] - best) * inv_t);
       if (target < run) { pick = i; break; }
     }
     out[r] = pick;
+    if (mirror != nullptr) *reinterpret_cast<volatile int*>(mirror + 2 + r) = pick;
   }
+  // not-a-number everywhere: nothing is drawn, `out` keeps what it held, and whoever watches the mirror learns that
+  if (chosen < 0 && mirror != nullptr && threadIdx.x == 0) *reinterpret_cast<volatile int*>(mirror + 2 + r) = out[r];
 }
 
 }  // namespace kvcm
@@ -241,14 +264,19 @@ KVCM_API int kvcm_argmax_f32(const float* logits, int* out, int rows, int vocab,
   return kvcm_argmax_status_f32(logits, out, rows, vocab, nullptr, stream);
 }
 
+KVCM_API int kvcm_sample_mirror_f32(const float* logits, const float* temperature, const unsigned long long* seed,
+                                    const long long* request_id, const int* position, int* out, int rows,
+                                    int vocab, int* status, int* mirror, void* stream) {
+  if (rows == 0) return 0;
+  if (mirror != nullptr && status == nullptr) return KVCM_ERR_UNSUPPORTED;
+  return pdl_launch(sample_kernel, dim3(rows), dim3(kSampleThreads), 0, (cudaStream_t)stream, logits, temperature, seed,
+                    request_id, position, out, vocab, status ? status_words() : StatusWords{}, status, mirror);
+}
+
 KVCM_API int kvcm_sample_status_f32(const float* logits, const float* temperature, const unsigned long long* seed,
                                     const long long* request_id, const int* position, int* out, int rows,
                                     int vocab, int* status, void* stream) {
-  if (rows == 0) return 0;
-  sample_kernel<<<rows, kSampleThreads, 0, (cudaStream_t)stream>>>(logits, temperature, seed, request_id, position,
-                                                                   out, vocab, status ? status_words() : StatusWords{},
-                                                                   status);
-  return KVCM_LAUNCH_RESULT();
+  return kvcm_sample_mirror_f32(logits, temperature, seed, request_id, position, out, rows, vocab, status, nullptr, stream);
 }
 
 KVCM_API int kvcm_sample_f32(const float* logits, const float* temperature,

@@ -17,7 +17,7 @@ struct KvcmDeviceBackend {
   int (*fetch_ints)(const int* pinned_src, int* dst, long long ints, void* stream);
   int (*sample)(const float* logits, const float* temperature, const unsigned long long* seed,
                 const long long* request_id, const int* position, int* out, int rows, int vocab, int* status,
-                void* stream);
+                int* mirror, void* stream);
   int (*copy_to_device)(void* dst, const void* src, size_t bytes, void* stream);
   int (*copy_to_host)(void* dst, const void* src, size_t bytes, void* stream);
   int (*stream_create)(void** stream);

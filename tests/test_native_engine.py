@@ -70,6 +70,22 @@ def test_tokens_do_not_depend_on_batching_and_every_step_runs_once(graphs, looka
     assert c.prefill_tokens == sum(len(p) for p in prompts) and c.preemptions == 0
 
 
+def test_requests_with_a_temperature_are_looked_ahead_too():
+    """(The stand-in device's draw is its argmax.)  Batches in which some or all requests sample, with one that ends early."""
+    for temps in ([0.8, 0.7, 0.9], [0.0, 0.8, 0.0]):
+        kv, sched, eng = make(max_batched_tokens=64)
+        prompts, new = [[5, 9, 3], [8] * 6, [7, 1]], [30, 12, 30]
+        for j, p in enumerate(prompts):
+            sched.add_request(j, p, new[j], temps[j], 11, 0.0)
+        done = {}
+        while not sched.idle():
+            eng.step()
+            for f in sched.take_finished():
+                done[f.id] = f
+        assert eng.lookahead_steps() > 15 and not eng.in_flight()
+        assert [done[j].generated() for j in range(3)] == [expected(p, n) for p, n in zip(prompts, new)]
+
+
 def test_lookahead_enqueues_the_next_step_before_this_one_is_read():
     """Steady greedy decoding: every call returns one step while the next is already on the device
     (the stand-in device runs a step when it is enqueued, so "on the device" shows as a forward call
