@@ -50,9 +50,10 @@ class NativeForward:
         # engine's limits (requests x heads x partitions x (head_dim + 2) floats, 64 partitions)
         self.attn_scratch = None if self.f32 else torch.empty(
             min(runner.max_seqs, 1024) * self.nh * 64 * (self.hd + 2), dtype=torch.float32, device=dev)
-        # partial sums of squares of the residual, one per 16 columns and row (None = norms are launches)
+        # partial sums of squares of the residual, per 16 columns and at most 16 rows or per 128 columns and at most 128
+        # rows (None = norms are launches)
         fuse = runner.options.get("fuse_norms", True) and not self.f32
-        self.norm_partials = torch.zeros((self.H + 15) // 16 * 16, dtype=torch.float32, device=dev) if fuse else None
+        self.norm_partials = torch.zeros((self.H + 127) // 128 * 128, dtype=torch.float32, device=dev) if fuse else None
         # cosines and sines of a step's angles, computed once a step for all layers (steps of many rows)
         self.rope_table = None if self.f32 else torch.empty(runner.max_rows * self.hd, dtype=torch.float32, device=dev)
         self.calls = 0
@@ -125,7 +126,7 @@ class NativeForward:
     def takes(self, ctx: StepContext) -> bool:
         o = ctx.options
         return (o.get("native_forward", True) and o.get("gemm", "auto") == "auto"
-                and not any(k in o for k in FORCING_OPTIONS) and ctx.tile_rows == 64)
+                and not any(o.get(k, "auto") != "auto" for k in FORCING_OPTIONS) and ctx.tile_rows == 64)
 
     def run(self, ctx: StepContext) -> Optional[torch.Tensor]:
         """Float32 logits [wanted rows, vocab] (None when no row is wanted).  Only enqueues device work."""
