@@ -107,7 +107,6 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   __shared__ uint32_t tmem_base;
   __shared__ volatile int abort_flag;
 
-  pdl_launch_dependents();
   // Later tiles of a prompt see more keys: the blocks are ordered with the heads fastest and the
   // last tiles first, so all long blocks start at once and the short ones fill the tail.
   const int tile = int(gridDim.y) - 1 - int(blockIdx.y), head = blockIdx.x;
@@ -160,6 +159,9 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
   const uint32_t tmem = tmem_base;
+  // only now, with the tensor memory in hand: a dependent that takes some early would keep a block of this launch waiting
+  // for it, and itself waits for this launch
+  pdl_launch_dependents();
   pdl_wait();                                                  // q and this step's keys come from kernels before
 
   auto fail = [&](int code) {

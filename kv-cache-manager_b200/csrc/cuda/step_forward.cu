@@ -67,6 +67,14 @@ int kvcm_qkv_rope_cache_scaled_bf16(const void*, const float*, int, float, const
                                     const int*, const float*, const int*, void*, void*, int, int, int, int, int, void*);
 int kvcm_gate_up_silu_scaled_bf16(const void*, const float*, int, float, const void*, void*, int, int, int, int, int, int, int,
                                   void*);
+int kvcm_gemm_tcgen05_splitk_supports(int, int, int, int, int);
+int kvcm_gemm_tcgen05_splitk_bf16(const void*, const void*, void*, int, int, int, int, int, int, int, void*);
+int kvcm_splitk_fused_supports(int, int, int);
+long long kvcm_splitk_norm_floats(int);
+int kvcm_splitk_residual_bf16(const void*, const void*, float*, float*, void*, const void*, int, int, int, int, int, int, int, void*);
+int kvcm_splitk_qkv_bf16(const void*, const float*, int, float, const void*, void*, int, int, int, int, int, const float*,
+                         const int*, void*, void*, int, int, int, int, void*);
+int kvcm_splitk_gate_up_silu_bf16(const void*, const float*, int, float, const void*, void*, int, int, int, int, int, int, void*);
 int kvcm_gate_up_silu_tcgen05_bf16(const void*, const void*, void*, int, int, int, int, int, int, void*);
 }
 
@@ -81,6 +89,11 @@ constexpr int kRopeTableMinRows = 64;                   // from here on the angl
 // Most rows of a step whose norms ride in its products (a decode step of the 1.1B shape, with and
 // without: 1 row 881 -> 809 us, 4 rows 902 -> 837, 8 rows 916 -> 869, 16 rows 1171 -> 1180).
 constexpr int kNormRideMaxRows = 8;
+// Rows of a step whose products run split over K on the tensor cores, norms, rotary encoding and activation in their
+// ends (gemm_tcgen05_splitk.cu).  The products of a layer of the 1.1B shape in us, against the library's (up to 16 rows the
+// streaming kernel's) with the separate kernels: 16 rows 31 against 36, 32 rows 35 against 43, 64 rows 42 against 45, 128 rows
+// 56 against 45.
+constexpr int kSplitkMinRows = 9, kSplitkMaxRows = 64;
 
 }  // namespace
 
@@ -124,6 +137,9 @@ int product(const KvcmForwardArgs& a, const void* x, const void* w, void* y, int
   if (a.f32) return kvcm_gemm_f32(x, w, y, M, N, K, K, K, N, 1, s);
   if ((M <= 8 || (long long)N * K * 2 <= kStreamMaxBytes) && kvcm_gemm_stream_supports(M, N, K))
     return kvcm_gemm_stream_bf16(x, w, y, M, N, K, K, K, N, out_f32 ? 1 : 0, a.sm_count, s);
+  if (M <= kSplitkMaxRows && kvcm_gemm_tcgen05_splitk_supports(M, N, K, K, K) &&
+      ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) == 0)
+    return kvcm_gemm_tcgen05_splitk_bf16(x, w, y, M, N, K, K, K, N, out_f32 ? 1 : 0, s);
   return library_gemm(a, x, w, y, M, N, K, out_f32, s);
 }
 
@@ -225,6 +241,19 @@ KVCM_API int kvcm_forward(const KvcmForwardArgs* ap, int* launches, void* stream
   };
   const bool may_ride = !a.f32 && a.norm_partials != nullptr && a.norm_partials_floats >= (long long)ss_tiles * 16 &&
                         T <= kNormRideMaxRows;
+  // A few dozen rows: the same on the tensor cores, every product of the step or none.
+  const auto aligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+  bool split = !a.f32 && a.norm_partials != nullptr && a.norm_partials_floats >= kvcm_splitk_norm_floats(H) &&
+               T >= kSplitkMinRows && T <= kSplitkMaxRows && a.rope_table != nullptr && a.rope_table_floats >= (long long)T * a.hd &&
+               (a.hd == 16 || a.hd == 32 || a.hd == 64 || a.hd == 128) && (H % 8) == 0 && (I % 8) == 0 && (QK % 8) == 0 &&
+               kvcm_splitk_fused_supports(T, H, QK) && kvcm_splitk_fused_supports(T, H, I) && kvcm_splitk_fused_supports(T, I, H) &&
+               aligned(a.x) && aligned(a.h) && aligned(a.qkv) && aligned(a.attn) && aligned(a.act) && aligned(a.rope_table);
+  for (int l = 0; l < a.num_layers; ++l) {
+    const KvcmForwardLayer& L = a.layers[l];
+    split = split && L.writes && aligned(L.w_qkv) && aligned(L.w_o) && aligned(L.w_gate_up) && aligned(L.w_down) &&
+            aligned(L.k_cache) && aligned(L.v_cache);
+  }
+  const int split_tiles = (H + 127) / 128;
   // (each sublayer by itself: where the down product is too wide for the streaming kernel, as at the
   // Llama-3-8B shape, the attention sublayer still closes this way)
   const bool ride_attn = may_ride && streams(H, QK), ride_ffn = may_ride && streams(H, I);
@@ -236,12 +265,17 @@ KVCM_API int kvcm_forward(const KvcmForwardArgs* ap, int* launches, void* stream
   KVCM_TRY(embed(a.tokens, a.embed, a.x, T, H, a.V, s)); ++n;
   bool table_filled = false;                            // the step's cosines and sines are in a.rope_table
   const void* pending = nullptr;                        // a sublayer's result not yet added to the residual
+  if (split) { KVCM_TRY(kvcm_rope_table_f32(a.positions, a.inv_freq, T, a.hd / 2, a.rope_table, s)); ++n; }
   bool handed = false;                                  // a.h and norm_partials hold the next norm's row before its scale
   // ends a sublayer: x += y w^T, one way or the other (next_norm: the norm weight of the product
   // that follows, where that product takes the scaled form)
   const auto close_sublayer = [&](const void* y, const void* w, int K, const void* next_norm, bool ride) {
     pending = nullptr;
     handed = false;
+    if (split) {
+      handed = next_norm != nullptr;
+      return kvcm_splitk_residual_bf16(y, w, a.x, a.norm_partials, a.h, next_norm, T, H, K, K, K, H, H, s);
+    }
     if (ride) {
       handed = next_norm != nullptr;
       return kvcm_gemm_stream_residual_bf16(y, w, a.x, a.norm_partials, a.h, next_norm, T, H, K, K, K, H, H, a.sm_count, s);
@@ -256,7 +290,12 @@ KVCM_API int kvcm_forward(const KvcmForwardArgs* ap, int* launches, void* stream
     const void* q = a.qkv;
     int q_stride = QKV;
     if (!handed) { KVCM_TRY(rmsnorm(a.x, pending, L.norm1, 0, a.h, nullptr, T, H, L.eps1, s)); ++n; }
-    if (qkv_fused(L)) {
+    if (split) {
+      KVCM_TRY(kvcm_splitk_qkv_bf16(a.h, handed ? a.norm_partials : nullptr, split_tiles, L.eps1, L.w_qkv, a.qkv, T, H, H, H, QK,
+                                    a.rope_table, a.group_slots[L.group], L.k_cache, L.v_cache, a.nh, a.nkv, a.hd, a.block_size, s));
+      ++n;
+      q_stride = QK;
+    } else if (qkv_fused(L)) {
       KVCM_TRY(kvcm_qkv_rope_cache_scaled_bf16(a.h, handed ? a.norm_partials : nullptr, ss_tiles, L.eps1, L.w_qkv, a.qkv, T, H,
                                                H, H, QK, a.positions, a.inv_freq, a.group_slots[L.group], L.k_cache,
                                                L.v_cache, a.nh, a.nkv, a.hd, a.block_size, a.sm_count, s));
@@ -280,10 +319,14 @@ KVCM_API int kvcm_forward(const KvcmForwardArgs* ap, int* launches, void* stream
       ++n;
     }
     KVCM_TRY(attention(a, L, q, q_stride, n, s));
-    KVCM_TRY(close_sublayer(a.attn, L.w_o, QK, gate_fused ? L.norm2 : nullptr, ride_attn)); ++n;
+    KVCM_TRY(close_sublayer(a.attn, L.w_o, QK, split || gate_fused ? L.norm2 : nullptr, ride_attn)); ++n;
     // feed-forward: gate/up product and activation -- one kernel where one exists for the shape
     if (!handed) { KVCM_TRY(rmsnorm(a.x, pending, L.norm2, 0, a.h, nullptr, T, H, L.eps2, s)); ++n; }
-    if (gate_fused) {
+    if (split) {
+      KVCM_TRY(kvcm_splitk_gate_up_silu_bf16(a.h, handed ? a.norm_partials : nullptr, split_tiles, L.eps2, L.w_gate_up, a.act, T, I,
+                                             H, H, H, I, s));
+      ++n;
+    } else if (gate_fused) {
       KVCM_TRY(kvcm_gate_up_silu_scaled_bf16(a.h, handed ? a.norm_partials : nullptr, ss_tiles, L.eps2, L.w_gate_up, a.act, T,
                                              I, H, H, H, I, a.sm_count, s));
       ++n;
@@ -294,7 +337,7 @@ KVCM_API int kvcm_forward(const KvcmForwardArgs* ap, int* launches, void* stream
       KVCM_TRY(product(a, a.h, L.w_gate_up, a.gate_up, T, 2 * I, H, false, s)); ++n;
       KVCM_TRY(silu_mul(a.gate_up, a.act, T, I, s)); ++n;
     }
-    const bool next_takes = l + 1 < a.num_layers && qkv_fused(a.layers[l + 1]);
+    const bool next_takes = l + 1 < a.num_layers && (split || qkv_fused(a.layers[l + 1]));
     KVCM_TRY(close_sublayer(a.act, L.w_down, I, next_takes ? a.layers[l + 1].norm1 : nullptr, ride_ffn)); ++n;
   }
   if (a.num_logits > 0) {

@@ -24,8 +24,8 @@ struct KvcmForwardArgs {
   const int* group_tables[KVCM_FORWARD_MAX_GROUPS]; const int* group_slots[KVCM_FORWARD_MAX_GROUPS];
   // buffers of the caller, sized for the step: x [T,H] float; h, proj [T,H]; qkv [T,QKV]; attn [T,nh*hd];
   // gate_up [T,2I]; act [T,I]; h_last [L,H]; logits [L,V] float; attn_scratch floats; a library workspace;
-  // norm_partials: ceil(H/16)*16 floats, or null = every norm is a launch of its own (with it, a step
-  // of at most 8 rows adds the residual and takes the norms inside its products)
+  // norm_partials: ceil(H/128)*128 floats, or null = every norm is a launch of its own (with it, a step
+  // of at most 64 rows adds the residual and takes the norms inside its products)
   float* x; void* h; void* qkv; void* attn; void* proj; void* gate_up; void* act; void* h_last; float* logits;
   // rope_table: rows x hd floats, or null = every layer's rotary kernel computes its angles itself
   float* attn_scratch; void* lib_workspace; float* norm_partials; float* rope_table;

@@ -373,6 +373,84 @@ def test_tcgen05_splitk_gemm(M, N, Kd):
     assert torch.equal(y, y2)
 
 
+@pytest.mark.parametrize("M,H,Kd,I,nh,nkv,hd,B", [(9, 64, 72, 20, 3, 1, 16, 8), (64, 2048, 2048, 5632, 32, 4, 64, 16),
+                                                   (33, 516, 1000, 132, 5, 2, 32, 4), (128, 4096, 512, 264, 4, 4, 128, 16), (1, 8, 8, 4, 1, 1, 64, 1)])
+def test_fused_ends_of_the_splitk_product(M, H, Kd, I, nh, nkv, hd, B):
+    """Residual, rotary + cache write and gated activation as the ends of the split-K product: the bits of the separate
+    kernels where the product is cut alike, the tolerance of the products against float64."""
+    import ctypes
+    lib, L = K(), K()._lib()
+    st, f = lib._stream(), ctypes.c_float
+
+    def call(name, *args):
+        args = [ctypes.c_void_p(None if a is None else a.data_ptr()) if a is None or torch.is_tensor(a) else a for a in args]
+        assert getattr(L, name)(*args, st) == 0
+        assert lib.splitk_error() == 0
+
+    g = torch.Generator().manual_seed(M + H)
+    y = torch.randn(M, Kd, generator=g).to(torch.bfloat16).to(DEV)
+    w = (torch.randn(H, Kd, generator=g) * 0.05).to(torch.bfloat16).to(DEV)
+    norm_w = (1.0 + 0.1 * torch.randn(H, generator=g)).to(torch.bfloat16).to(DEV)
+    resid0 = (3.0 * torch.randn(M, H, generator=g)).to(DEV)
+    proj = torch.empty(M, H, dtype=torch.bfloat16, device=DEV)
+    lib.gemm_tcgen05_splitk(y, w, proj)
+    L.kvcm_splitk_norm_floats.restype = ctypes.c_longlong
+    tiles = (H + 127) // 128
+    assert L.kvcm_splitk_norm_floats(H) == tiles * 128
+    resid, ss = resid0.clone(), torch.full((tiles, 128), float("nan"), device=DEV)
+    h = torch.full((M, H), float("nan"), dtype=torch.bfloat16, device=DEV)
+    call("kvcm_splitk_residual_bf16", y, w, resid, ss, h, norm_w, M, H, Kd, Kd, Kd, H, H)
+    assert torch.equal(resid, resid0 + proj.float()) and torch.equal(h, (norm_w.float() * resid).to(torch.bfloat16))
+    x64 = resid.double()
+    assert torch.allclose(ss[:, :M].double().sum(0), (x64 ** 2).sum(1), rtol=1e-5)
+    again, ss2 = resid0.clone(), torch.zeros_like(ss)
+    call("kvcm_splitk_residual_bf16", y, w, again, ss2, None, None, M, H, Kd, Kd, Kd, H, H)      # nothing handed on
+    assert torch.equal(again, resid) and torch.equal(ss2[:, :M], ss[:, :M])
+    if H % 8:
+        return                                                        # (no product reads rows of this width)
+    eps = 1e-5
+    normed = norm_w.double() * x64 * torch.rsqrt((x64 ** 2).mean(1, keepdim=True) + eps)
+    # gate/up: unscaled against the separate kernels, scaled against float64
+    wg = (torch.randn(2 * I, H, generator=g) * 0.05).to(torch.bfloat16).to(DEV)
+    a1, a2 = (torch.full((M, I), float("nan"), dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    call("kvcm_splitk_gate_up_silu_bf16", h, None, 0, f(0), wg, a1, M, I, H, H, H, I)
+    gg = h.double() @ wg.double().T
+    close(a1, (gg[:, :I] * torch.sigmoid(gg[:, :I]) * gg[:, I:]).cpu(), "bfloat16", "gate/up")
+    if I % 64 == 0:
+        gu = torch.empty(M, 2 * I, dtype=torch.bfloat16, device=DEV)
+        lib.gemm_tcgen05_splitk(h, wg, gu)
+        lib.silu_mul(gu, a2)
+        assert torch.equal(a1, a2)
+    call("kvcm_splitk_gate_up_silu_bf16", h, ss, tiles, f(eps), wg, a2, M, I, H, H, H, I)
+    gg = normed @ wg.double().T
+    close(a2, (gg[:, :I] * torch.sigmoid(gg[:, :I]) * gg[:, I:]).cpu(), "bfloat16", "scaled gate/up")
+    # qkv with the angles of the step from their table
+    heads = nh + 2 * nkv
+    wq = (torch.randn(heads * hd, H, generator=g) * 0.05).to(torch.bfloat16).to(DEV)
+    pos = torch.randint(0, 3000, (M,), generator=g).to(torch.int32).to(DEV)
+    pages = (M + B - 1) // B + 3
+    slots = torch.randperm(pages * B, generator=g)[:M].to(torch.int32)
+    if M > 2:
+        slots[1] = -1
+    slots = slots.to(DEV)
+    inv = (10000.0 ** (-2.0 * torch.arange(hd // 2, dtype=torch.float64) / hd)).float().to(DEV)
+    table = torch.empty(M, hd, device=DEV)
+    lib.rope_table(pos, inv, table)
+    qkv = torch.empty(M, heads * hd, dtype=torch.bfloat16, device=DEV)
+    lib.gemm_tcgen05_splitk(h, wq, qkv)
+    k1 = torch.zeros(pages, nkv, B, hd, dtype=torch.bfloat16, device=DEV)
+    v1, k2, v2 = torch.zeros_like(k1), torch.zeros_like(k1), torch.zeros_like(k1)
+    lib.rope_cache_table(qkv, table, slots, k1, v1, nh, nkv, hd, B, True)
+    q = torch.full((M, nh * hd), float("nan"), dtype=torch.bfloat16, device=DEV)
+    call("kvcm_splitk_qkv_bf16", h, None, 0, f(0), wq, q, M, H, H, H, nh * hd, table, slots, k2, v2, nh, nkv, hd, B)
+    assert torch.equal(q, qkv[:, :nh * hd]) and torch.equal(k2, k1) and torch.equal(v2, v1)
+    call("kvcm_splitk_qkv_bf16", h, ss, tiles, f(eps), wq, q, M, H, H, H, nh * hd, table, slots, k2, v2, nh, nkv, hd, B)
+    live = (slots >= 0).cpu()
+    sl = slots.cpu().long()[live]
+    vref = (normed @ wq.double().T)[:, (nh + nkv) * hd:].reshape(M, nkv, hd).cpu()[live]
+    close(v2.cpu()[sl // B, :, sl % B], vref, "bfloat16", "v rows of the scaled product")
+
+
 @pytest.mark.parametrize("M,H,I", [(2048, 2048, 5632), (300, 96, 1000), (129, 64, 24), (640, 256, 128)])
 def test_tcgen05_gate_up_with_the_activation_in_its_epilogue(M, H, I):
     """Bit for bit the tcgen05 product followed by the activation kernel, and close to float64."""
