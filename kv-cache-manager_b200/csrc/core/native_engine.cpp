@@ -194,13 +194,10 @@ int NativeEngine::run_device(const KvcmForwardArgs& a, int logit_rows, bool temp
   int launches = 0, extra = 0;
   const size_t R = sampling_rows(logit_rows);
   if (fetch_from != nullptr) {
-    check(dev_.fetch_ints(fetch_from, fetch_to, fetch_ints, stream_), "fetching the batch");
+    check(dev_.fetch_ints(fetch_from, fetch_to, fetch_ints, reinterpret_cast<const int*>(fetch_sampling),
+                          reinterpret_cast<int*>(d_sampling_), fetch_sampling != nullptr ? (long long)(6 * R) : 0, stream_),
+          "fetching the batch");
     extra = 1;
-  }
-  if (fetch_sampling != nullptr) {
-    check(dev_.fetch_ints(reinterpret_cast<const int*>(fetch_sampling), reinterpret_cast<int*>(d_sampling_), (long long)(6 * R), stream_),
-          "fetching the sampling parameters");
-    ++extra;
   }
   check(dev_.forward(&a, &launches, stream_), "the forward pass");
   launches += extra;
@@ -584,9 +581,13 @@ int fake_argmax(const float* logits, int* out, int rows, int vocab, int* status,
   else fake_argmax_now(logits, out, rows, vocab, status, mirror);
   return 0;
 }
-int fake_fetch_ints(const int* src, int* dst, long long ints, void*) {
-  if (g_fake.recording) g_fake.open->calls.push_back([=] { std::memcpy(dst, src, size_t(ints) * 4); });
-  else std::memcpy(dst, src, size_t(ints) * 4);
+int fake_fetch_ints(const int* src, int* dst, long long ints, const int* src2, int* dst2, long long ints2, void*) {
+  const auto fetch = [=] {
+    std::memcpy(dst, src, size_t(ints) * 4);
+    if (ints2 > 0) std::memcpy(dst2, src2, size_t(ints2) * 4);
+  };
+  if (g_fake.recording) g_fake.open->calls.push_back(fetch);
+  else fetch();
   return 0;
 }
 int fake_sample(const float* logits, const float*, const unsigned long long*, const long long*, const int*, int* out,

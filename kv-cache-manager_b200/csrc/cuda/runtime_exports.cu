@@ -11,7 +11,7 @@
 extern "C" {
 int kvcm_forward(const KvcmForwardArgs*, int*, void*);
 int kvcm_argmax_mirror_f32(const float*, int*, int, int, int*, int*, void*);
-int kvcm_fetch_ints(const int*, int*, long long, void*);
+int kvcm_fetch_ints(const int*, int*, long long, const int*, int*, long long, void*);
 int kvcm_sample_mirror_f32(const float*, const float*, const unsigned long long*, const long long*, const int*, int*, int, int,
                            int*, int*, void*);
 int kvcm_stream_error(void);

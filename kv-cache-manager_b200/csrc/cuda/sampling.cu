@@ -167,12 +167,17 @@ sample_kernel(const float* __restrict__ logits, const float* __restrict__ temper
     last_filled = -1;
     const int filled = (vocab + seg - 1) / seg;
     float run = 0.f;
-    for (int i = 0; i < filled; i += 4) {                    // (part[] is zero beyond the last segment)
-      const float4 t = *reinterpret_cast<const float4*>(part + i);
-      float4 u;
-      u.x = run + t.x; u.y = u.x + t.y; u.z = u.y + t.z; u.w = u.z + t.w;
-      *reinterpret_cast<float4*>(upto + i) = u;
-      run = u.w;
+    for (int i0 = 0; i0 < filled; i0 += 32) {                // (part[] is zero beyond the last segment)
+      float4 t[8];                                           // eight reads in flight: the additions are the chain, not these
+#pragma unroll
+      for (int k = 0; k < 8; ++k) t[k] = *reinterpret_cast<const float4*>(part + i0 + 4 * k);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        float4 u;
+        u.x = run + t[k].x; u.y = u.x + t[k].y; u.z = u.y + t[k].z; u.w = u.z + t[k].w;
+        *reinterpret_cast<float4*>(upto + i0 + 4 * k) = u;
+        run = u.w;
+      }
     }
     total = run;
   }
@@ -244,19 +249,29 @@ namespace kvcm {
 // read: a kernel that fetches them itself, as the first launch of a recorded decode step, instead
 // of a copy command in front of it (a copy engine needs several microseconds to start, in which the
 // SMs would idle).
-__global__ void __launch_bounds__(256) fetch_ints_kernel(const int4* __restrict__ src, int4* __restrict__ dst, int vecs) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < vecs; i += gridDim.x * blockDim.x) dst[i] = src[i];
+// (With a second array, the sampling parameters: one trip to the host for both, 4.4 us each otherwise.)
+__global__ void __launch_bounds__(256) fetch_ints_kernel(const int4* __restrict__ src, int4* __restrict__ dst, int vecs,
+                                                         const int4* __restrict__ src2, int4* __restrict__ dst2, int vecs2) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < vecs + vecs2; i += gridDim.x * blockDim.x) {
+    if (i < vecs) dst[i] = src[i];
+    else dst2[i - vecs] = src2[i - vecs];
+  }
 }
 }  // namespace kvcm
 
-// `ints` a multiple of 4 (the batch builder pads every array to 16 bytes); both addresses 16-byte aligned.
-KVCM_API int kvcm_fetch_ints(const int* pinned_src, int* dst, long long ints, void* stream) {
+// `ints`, `ints2` multiples of 4 (the batch builder pads every array to 16 bytes); all addresses 16-byte aligned.  The second
+// array is optional (ints2 = 0).
+KVCM_API int kvcm_fetch_ints(const int* pinned_src, int* dst, long long ints, const int* pinned_src2, int* dst2, long long ints2,
+                             void* stream) {
   if (ints <= 0) return 0;
-  if ((ints & 3) || (reinterpret_cast<uintptr_t>(pinned_src) & 15) || (reinterpret_cast<uintptr_t>(dst) & 15))
+  if (ints2 < 0 || ((ints | ints2) & 3) ||
+      ((reinterpret_cast<uintptr_t>(pinned_src) | reinterpret_cast<uintptr_t>(dst)) & 15) ||
+      (ints2 > 0 && ((reinterpret_cast<uintptr_t>(pinned_src2) | reinterpret_cast<uintptr_t>(dst2)) & 15)))
     return KVCM_ERR_UNSUPPORTED;
-  const int vecs = int(ints / 4);
-  fetch_ints_kernel<<<std::min((vecs + 255) / 256, 8), 256, 0, (cudaStream_t)stream>>>(
-      reinterpret_cast<const int4*>(pinned_src), reinterpret_cast<int4*>(dst), vecs);
+  const int vecs = int(ints / 4), vecs2 = int(ints2 / 4);
+  fetch_ints_kernel<<<std::min((vecs + vecs2 + 255) / 256, 8), 256, 0, (cudaStream_t)stream>>>(
+      reinterpret_cast<const int4*>(pinned_src), reinterpret_cast<int4*>(dst), vecs, reinterpret_cast<const int4*>(pinned_src2),
+      reinterpret_cast<int4*>(dst2), vecs2);
   return KVCM_LAUNCH_RESULT();
 }
 

@@ -13,8 +13,10 @@ struct KvcmDeviceBackend {
   int (*forward)(const KvcmForwardArgs* args, int* launches, void* stream);
   // `mirror` (optional): pinned host memory [2 + rows] that the device also writes [status pair | tokens] into
   int (*argmax)(const float* logits, int* out, int rows, int vocab, int* status, int* mirror, void* stream);
-  // the batch's integer arrays fetched from pinned host memory by a kernel (ints a multiple of 4)
-  int (*fetch_ints)(const int* pinned_src, int* dst, long long ints, void* stream);
+  // the batch's integer arrays, and a second array where ints2 > 0, fetched from pinned host memory by a kernel (ints,
+  // ints2 multiples of 4)
+  int (*fetch_ints)(const int* pinned_src, int* dst, long long ints, const int* pinned_src2, int* dst2, long long ints2,
+                    void* stream);
   int (*sample)(const float* logits, const float* temperature, const unsigned long long* seed,
                 const long long* request_id, const int* position, int* out, int rows, int vocab, int* status,
                 int* mirror, void* stream);
