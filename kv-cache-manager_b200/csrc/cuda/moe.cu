@@ -15,14 +15,18 @@
 //   down     y[pair]   = act[pair] Wd_e^T                           per tile, float results
 //   combine  out[row]  = sum_k weight[row, k] * y[row, k] + gate[row] * shared[row]   (float)
 // (bfloat16 rows whose sizes allow it take the tensor-core form of the two products,
-// csrc/cuda/moe_tcgen05.cu, after the same sort into tiles of 128.)
+// csrc/cuda/moe_tcgen05.cu, after the same sort into tiles of 128; steps of a few rows the form without a sort,
+// csrc/cuda/moe_few.cu.)
 //
 // Nothing is read on the host: counts and tile lists stay on the device and the product grids
 // are sized for the worst case (pairs / 64 + experts tiles), so a step can be recorded into a
 // CUDA graph.  Every output element is accumulated by one thread over k in ascending order, so
 // a row's result does not depend on what else is in the batch or on the order inside a tile.
 // Instantiated for float (the true 32-bit path: float FMAs only) and bfloat16 storage.
+#include <cooperative_groups.h>
+
 #include "common.cuh"
+#include "pdl.cuh"
 
 namespace kvcm {
 
@@ -292,6 +296,8 @@ __global__ void __launch_bounds__(ROUTE_WARPS * 32)
 moe_route_mma_kernel(const bf16* __restrict__ h, int ldh, const bf16* __restrict__ wr, int rows, int D, RouteChoice choice) {
   constexpr int NP = 8 * NT;
   extern __shared__ float route_smem[];
+  pdl_launch_dependents();
+  pdl_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t4 = lane & 3;
   const int row0 = blockIdx.x * ROUTE_MMA_ROWS;
   const int E = choice.E, outs = E + (choice.has_gate ? 1 : 0);
@@ -344,6 +350,82 @@ moe_route_mma_kernel(const bf16* __restrict__ h, int ldh, const bf16* __restrict
     const int row = row0 + rr;
     if (row < rows) route_choose(choice, route_smem + rr * zstride, row, lane);
   }
+}
+
+// The same for a step of few rows, which one block would walk through in one latency after another: the width is split
+// over the eight blocks of a cluster, so that at a width of 2,048 every warp has one block of 32 columns, whose router rows it
+// asks for before the dependency wait (they are weights).  The blocks' sums (over their warps in order) meet in distributed
+// shared memory; block r adds them in the order of the blocks and chooses for rows r and r + 8.  At most 8 * NT outputs.
+// Four rows of 2,048 columns, 33 outputs, in a decode step: 6.9 us, one block of eight warps 12.8.
+constexpr int ROUTE_SPLIT = 8;
+template <int NT>
+__global__ void __launch_bounds__(ROUTE_WARPS * 32)
+moe_route_few_kernel(const bf16* h, int ldh, const bf16* __restrict__ wr, int rows, int D, RouteChoice choice) {
+  constexpr int NP = 8 * NT;
+  extern __shared__ __align__(16) float route_smem[];       // [2] rows of a choice | [warps][16][NP] | [16][NP]
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t4 = lane & 3;
+  const int row0 = int(blockIdx.x) / ROUTE_SPLIT * ROUTE_MMA_ROWS, rank = int(blockIdx.x) % ROUTE_SPLIT;
+  const int E = choice.E, outs = E + (choice.has_gate ? 1 : 0);
+  const int zstride = (2 * E + 1 + choice.G + 3) & ~3;
+  float* part = route_smem + 2 * zstride;
+  float* sums = part + ROUTE_WARPS * ROUTE_MMA_ROWS * NP;
+  const uint4 none = make_uint4(0u, 0u, 0u, 0u);
+  float acc[NT][4];
+  const bf16* we[NT];
+#pragma unroll
+  for (int i = 0; i < NT; ++i) {
+    acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+    we[i] = wr + size_t(min(8 * i + g, outs - 1)) * D + t4 * 8;
+  }
+  const bf16* ra = h + size_t(min(row0 + g, rows - 1)) * ldh + t4 * 8;
+  const bf16* rb = h + size_t(min(row0 + g + 8, rows - 1)) * ldh + t4 * 8;
+  pdl_launch_dependents();
+  bool waited = false;
+  for (int kb = (rank * ROUTE_WARPS + warp) * 32; kb < D; kb += ROUTE_SPLIT * ROUTE_WARPS * 32) {
+    const bool in = kb + t4 * 8 < D;                        // (D % 8 == 0)
+    uint4 w[NT];
+#pragma unroll
+    for (int i = 0; i < NT; ++i) w[i] = in ? *reinterpret_cast<const uint4*>(we[i] + kb) : none;
+    if (!waited) { pdl_wait(); waited = true; }
+    const uint4 a = in ? *reinterpret_cast<const uint4*>(ra + kb) : none, b = in ? *reinterpret_cast<const uint4*>(rb + kb) : none;
+#pragma unroll
+    for (int i = 0; i < NT; ++i) {
+      route_mma(acc[i], a.x, b.x, a.y, b.y, w[i].x, w[i].y);
+      route_mma(acc[i], a.z, b.z, a.w, b.w, w[i].z, w[i].w);
+    }
+  }
+  if (!waited) pdl_wait();                                  // before anything is written
+#pragma unroll
+  for (int i = 0; i < NT; ++i) {
+    float* at = part + (warp * ROUTE_MMA_ROWS + g) * NP + 8 * i + 2 * t4;
+    at[0] = acc[i][0]; at[1] = acc[i][1];
+    at[8 * NP] = acc[i][2]; at[8 * NP + 1] = acc[i][3];
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < ROUTE_MMA_ROWS * NP; i += ROUTE_WARPS * 32) {
+    float z = 0.f;
+#pragma unroll
+    for (int w = 0; w < ROUTE_WARPS; ++w) z += part[w * ROUTE_MMA_ROWS * NP + i];
+    sums[i] = z;
+  }
+  const auto cluster = cooperative_groups::this_cluster();
+  cluster.sync();
+  const int local = rank + ROUTE_SPLIT * warp, row = row0 + local;
+  if (warp < ROUTE_MMA_ROWS / ROUTE_SPLIT && row < rows) {
+    float* z = route_smem + warp * zstride;
+    for (int e = lane; e < outs; e += 32) {
+      float v[ROUTE_SPLIT];
+#pragma unroll
+      for (int r = 0; r < ROUTE_SPLIT; ++r) v[r] = *cluster.map_shared_rank(sums + local * NP + e, r);
+      float t = v[0];
+#pragma unroll
+      for (int r = 1; r < ROUTE_SPLIT; ++r) t += v[r];
+      z[e] = t;
+    }
+    __syncwarp();
+    route_choose(choice, z, row, lane);
+  }
+  cluster.sync();                                           // nobody leaves while its sums are read
 }
 
 // ------------------------------------------------------------------------------------- sort
@@ -504,16 +586,47 @@ moe_down_kernel(const T* __restrict__ act, const T* __restrict__ wd, const int* 
 }
 
 // out[row, i] = sum_k wt[row, k] * y[place_of[row * top + k], i]  (+ gate[row] * shared[row, i]),
-// the choices added in the order of k.
-template <typename T>
+// the choices added in the order of k.  A block takes 1,024 columns of a row, a thread four neighbours: the choices' pieces
+// are all under way at once (with a block a row and a column a thread they came one after another: 7.3 us at four rows of
+// 2,048 in a decode step, now 2.4).
+constexpr int kCombineAhead = 8;
+template <bool VEC>
 __global__ void __launch_bounds__(256)
 moe_combine_kernel(const float* __restrict__ y, const int* __restrict__ place_of, const float* __restrict__ wt, int top,
                    const float* __restrict__ shared_y, const float* __restrict__ gate, float* __restrict__ out, int D) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int row = blockIdx.x;
-  for (int i = threadIdx.x; i < D; i += blockDim.x) {
+  const int* place = place_of + size_t(row) * top;
+  const float* w = wt + size_t(row) * top;
+  if constexpr (VEC) {
+    const int i = (blockIdx.y * 256 + threadIdx.x) * 4;
+    if (i >= D) return;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f), sh = acc;
+    if (shared_y) sh = *reinterpret_cast<const float4*>(shared_y + size_t(row) * D + i);
+    for (int k0 = 0; k0 < top; k0 += kCombineAhead) {
+      float4 v[kCombineAhead];
+#pragma unroll
+      for (int u = 0; u < kCombineAhead; ++u)
+        if (k0 + u < top) v[u] = *reinterpret_cast<const float4*>(y + size_t(place[k0 + u]) * D + i);
+#pragma unroll
+      for (int u = 0; u < kCombineAhead; ++u)
+        if (k0 + u < top) {
+          const float f = w[k0 + u];
+          acc.x = fmaf(f, v[u].x, acc.x); acc.y = fmaf(f, v[u].y, acc.y);
+          acc.z = fmaf(f, v[u].z, acc.z); acc.w = fmaf(f, v[u].w, acc.w);
+        }
+    }
+    if (shared_y) {
+      const float f = gate ? gate[row] : 1.f;
+      acc.x += f * sh.x; acc.y += f * sh.y; acc.z += f * sh.z; acc.w += f * sh.w;
+    }
+    *reinterpret_cast<float4*>(out + size_t(row) * D + i) = acc;
+  } else {
+    const int i = blockIdx.y * 256 + threadIdx.x;
+    if (i >= D) return;
     float acc = 0.f;
-    for (int k = 0; k < top; ++k)
-      acc = fmaf(wt[size_t(row) * top + k], y[size_t(place_of[size_t(row) * top + k]) * D + i], acc);
+    for (int k = 0; k < top; ++k) acc = fmaf(w[k], y[size_t(place[k]) * D + i], acc);
     if (shared_y) acc += (gate ? gate[row] : 1.f) * shared_y[size_t(row) * D + i];
     out[size_t(row) * D + i] = acc;
   }
@@ -533,15 +646,21 @@ int launch_moe_route(const void* h, int ldh, const void* wr, int w_f32, int rows
   if (smem > 200 * 1024) return KVCM_ERR_UNSUPPORTED;
   const RouteChoice choice = {E, G, keep, top, has_gate, scores, group_top, renorm, scale, correction, bias, idx, wt, gate_out};
   if constexpr (sizeof(T) == 2) {
-    const int outs = E + (has_gate ? 1 : 0), np = outs <= 32 ? 32 : 64;
+    const int outs = E + (has_gate ? 1 : 0), np = outs <= 32 ? 32 : outs <= 40 ? 40 : 64;
     const size_t mma_smem = ROUTE_MMA_ROWS * (zstride + ROUTE_WARPS * np) * sizeof(float);
     if (!w_f32 && (D % 8) == 0 && (ldh % 8) == 0 && ((reinterpret_cast<uintptr_t>(h) | reinterpret_cast<uintptr_t>(wr)) & 15) == 0 &&
         mma_smem <= 200 * 1024) {
       const dim3 grid((rows + ROUTE_MMA_ROWS - 1) / ROUTE_MMA_ROWS);
-      auto kernel = np == 32 ? moe_route_mma_kernel<4> : moe_route_mma_kernel<8>;
+      const size_t few_smem = (2 * zstride + (ROUTE_WARPS + 1) * ROUTE_MMA_ROWS * np) * sizeof(float);
+      // up to four clusters; with more rows the blocks of sixteen fill SMs by themselves
+      if (rows <= 4 * ROUTE_MMA_ROWS && outs <= np && few_smem <= 48 * 1024) {
+        auto few = np == 32 ? moe_route_few_kernel<4> : np == 40 ? moe_route_few_kernel<5> : moe_route_few_kernel<8>;
+        return pdl_launch_cluster(few, dim3(grid.x * ROUTE_SPLIT), dim3(ROUTE_WARPS * 32), few_smem, s, ROUTE_SPLIT, (const bf16*)h, ldh,
+                                  (const bf16*)wr, rows, D, choice);
+      }
+      auto kernel = np == 32 ? moe_route_mma_kernel<4> : np == 40 ? moe_route_mma_kernel<5> : moe_route_mma_kernel<8>;
       if (mma_smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mma_smem);
-      kernel<<<grid, ROUTE_WARPS * 32, mma_smem, s>>>((const bf16*)h, ldh, (const bf16*)wr, rows, D, choice);
-      return KVCM_LAUNCH_RESULT();
+      return pdl_launch(kernel, grid, dim3(ROUTE_WARPS * 32), mma_smem, s, (const bf16*)h, ldh, (const bf16*)wr, rows, D, choice);
     }
   }
   const int vec = w_f32 ? 4 : RouteVec<T>::N;
@@ -662,6 +781,8 @@ KVCM_API int kvcm_moe_combine(const float* y, const int* work, const float* wt, 
                               const float* gate, float* out, int rows, int D, void* stream) {
   if (rows == 0) return 0;
   const int* place_of = work + E + 2 + rows * top;
-  moe_combine_kernel<float><<<rows, 256, 0, (cudaStream_t)stream>>>(y, place_of, wt, top, shared_y, gate, out, D);
-  return KVCM_LAUNCH_RESULT();
+  const bool vec = (D % 4) == 0 && ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(shared_y) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
+  const int per = vec ? 1024 : 256;
+  return pdl_launch(vec ? moe_combine_kernel<true> : moe_combine_kernel<false>, dim3(rows, (D + per - 1) / per), dim3(256), 0,
+                    (cudaStream_t)stream, y, place_of, wt, top, shared_y, gate, out, D);
 }

@@ -1139,6 +1139,31 @@ def moe_tcgen05_supported(expert_ff: int, hidden: int) -> bool:
     return bool(_lib().kvcm_moe_tcgen05_supports(int(expert_ff), int(hidden)))
 
 
+def moe_few_supported(h: torch.Tensor, top: int, experts: int, expert_ff: int) -> bool:
+    """A step of few bfloat16 rows: the experts' products without sorted pairs (csrc/cuda/moe_few.cu)."""
+    return (h.dtype == torch.bfloat16 and h.stride(1) == 1 and h.stride(0) % 8 == 0 and h.data_ptr() % 16 == 0
+            and bool(_lib().kvcm_moe_few_supports(h.shape[0], int(top), int(experts), int(expert_ff), h.shape[1])))
+
+
+def moe_experts_few(h: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tensor, idx: torch.Tensor,
+                    work: torch.Tensor, act: torch.Tensor, y: torch.Tensor) -> None:
+    """``moe_experts`` for a step of few rows (``moe_few_supported``): y in the order of the pairs, which ``work`` says too."""
+    _cuda(h, w_gate_up, w_down, idx, work, act, y)
+    T, D = h.shape
+    top = idx.shape[1]
+    E, F2, _ = w_gate_up.shape
+    F = F2 // 2
+    _need(w_gate_up.is_contiguous() and w_down.is_contiguous() and w_gate_up.shape == (E, 2 * F, D) and w_down.shape == (E, D, F)
+          and w_gate_up.dtype == h.dtype == w_down.dtype == act.dtype == torch.bfloat16, "moe_experts_few: weights")
+    _need(h.stride(1) == 1 and idx.dtype == _I32 and idx.is_contiguous() and act.is_contiguous() and act.shape == (T * top, F)
+          and y.dtype == torch.float32 and y.is_contiguous() and y.shape == (T * top, D), "moe_experts_few: buffers")
+    _need(work.dtype == _I32 and work.numel() >= moe_work_ints(T, top, E), "moe_experts_few: work too small")
+    global _launches
+    _check(_lib().kvcm_moe_experts_few_bf16(_p(h), h.stride(0), _p(w_gate_up), _p(w_down), _p(idx), T, top, E, F, D, _p(work),
+                                            _p(act), _p(y), _stream()), "moe_experts_few", f"(experts={E}, ff={F})")
+    _launches += 1                          # gate/up, down
+
+
 def moe_tcgen05_error() -> int:
     """Error word of the experts' tensor-core products: 0, or (code << 16 | block) of a bounded wait
     that ran out.  Reading clears it.  Synchronises the device."""

@@ -101,6 +101,9 @@ class RoutedExperts(FeedForward):
         work = torch.empty((K.moe_work_ints(M, top, self.experts),), dtype=torch.int32, device=dev)
         act = torch.empty((M * top, self.expert_ff), dtype=h.dtype, device=dev)
         y = torch.empty((M * top, D), dtype=torch.float32, device=dev)
+        if ctx.options.get("gemm", "auto") != "plain" and K.moe_few_supported(h, top, self.experts, self.expert_ff):
+            K.moe_experts_few(h, self._wgu, self._wd, idx, work, act, y)
+            return y, work, wt, gate
         xs = None
         if (h.dtype == torch.bfloat16 and ctx.options.get("gemm", "auto") != "plain"
                 and K.moe_tcgen05_supported(self.expert_ff, D) and h.stride(0) % 8 == 0):

@@ -466,6 +466,54 @@ def test_expert_products_on_tensor_cores_against_float64(T, E, top, F, D):
     assert (outs[0] - outs[1]).abs().max().item() <= 0.04 * ref.std().item()
 
 
+@pytest.mark.parametrize("T,E,top,F,D", [(1, 1, 1, 8, 8), (4, 32, 4, 512, 2048), (9, 5, 3, 72, 264), (13, 4, 2, 24, 40), (16, 16, 8, 40, 136),
+                                         (8, 6, 20, 264, 72), (3, 1000, 2, 16, 24)])
+def test_expert_products_of_few_rows_against_float64(T, E, top, F, D):
+    """The form without a sort: experts without a row, one that every row chose, and (top 20 of 6) rows that name an expert
+    more than once, which a choice among not-a-numbers gives.  The bound is that of the test above."""
+    from kvcm.kernels import library as K
+    g = torch.Generator().manual_seed(T + E)
+    h = (torch.randn(T, D + 8, generator=g) * 0.5).to(torch.bfloat16).cuda()[:, :D]            # strided rows
+    wgu = (torch.randn(E, 2 * F, D, generator=g) * D ** -0.5).to(torch.bfloat16).cuda()
+    wd = (torch.randn(E, D, F, generator=g) * F ** -0.5).to(torch.bfloat16).cuda()
+    idx = torch.randint(0, E, (T, top), generator=g) if top > E else torch.stack([torch.randperm(E, generator=g)[:top] for _ in range(T)])
+    idx[:, 0] = E - 1
+    wt, shared, gate = torch.rand(T, top, generator=g).cuda(), torch.randn(T, D, generator=g).cuda(), torch.rand(T, generator=g).cuda()
+    assert K.moe_few_supported(h, top, E, F)
+    work = torch.empty(K.moe_work_ints(T, top, E), dtype=torch.int32, device="cuda")
+    act = torch.empty(T * top, F, dtype=torch.bfloat16, device="cuda")
+    y = torch.full((T * top, D), float("nan"), device="cuda")
+    out = torch.empty(T, D, device="cuda")
+    K.moe_experts_few(h, wgu, wd, idx.to(torch.int32).cuda(), work, act, y)
+    K.moe_combine(y, work, wt, E, shared, gate, out)
+    hd, e = h.double(), idx.flatten().cuda()
+    rows = hd.repeat_interleave(top, 0)[:, None]
+    a = torch.bmm(rows, wgu[e].double().transpose(1, 2))[:, 0]
+    ref = torch.bmm((P.silu(a[:, :F]) * a[:, F:])[:, None], wd[e].double().transpose(1, 2))[:, 0]
+    assert (y.double() - ref).abs().max().item() <= 0.04 * ref.std(correction=0).item()
+    assert torch.allclose(out.double(), (wt.double()[..., None] * y.double().view(T, top, D)).sum(1) + gate.double()[:, None] * shared.double(), atol=1e-5)
+
+
+@pytest.mark.parametrize("T,E,D,gate", [(1, 8, 8, False), (4, 32, 2048, True), (16, 31, 72, False), (17, 39, 2056, True), (64, 60, 520, False)])
+def test_router_split_over_a_cluster_against_float64(T, E, D, gate):
+    """Softmax weights and choices of steps of few rows: the logits of both forms are float sums of exact products."""
+    from kvcm.kernels import library as K
+    g = torch.Generator().manual_seed(T * 7 + E)
+    h = torch.randn(T, D + 8, generator=g).to(torch.bfloat16).cuda()[:, :D]
+    wr = (torch.randn(E + gate, D, generator=g) * 3 * D ** -0.5).to(torch.bfloat16).cuda()
+    top = min(4, E)
+    idx = torch.full((T, top), -1, dtype=torch.int32, device="cuda")
+    wt = torch.empty(T, top, device="cuda")
+    out = torch.empty(T, device="cuda") if gate else None
+    K.moe_route(h, wr, E, 1, 1, top, 1.5, idx, wt, out)
+    z = h.double() @ wr.double().T
+    s = torch.softmax(z[:, :E], -1)
+    assert torch.equal(idx.long(), s.topk(top, -1).indices)
+    assert torch.allclose(wt.double(), 1.5 * s.gather(1, idx.long()), rtol=1e-4)
+    if gate:
+        assert torch.allclose(out.double(), torch.sigmoid(z[:, E]), rtol=1e-4)
+
+
 def test_score_borrows_a_state_slot(folders, oracle):
     """``Engine.score`` on a model with per-request state: teacher-forced logits of a whole sequence,
     twice (the slot is zeroed each time) and with requests running beside it."""
