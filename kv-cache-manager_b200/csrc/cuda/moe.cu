@@ -432,38 +432,89 @@ moe_route_few_kernel(const bf16* h, int ldh, const bf16* __restrict__ wr, int ro
 // One block.  offsets[e] = first sorted place of expert e; pair_of[place] = row * top + k and
 // place_of[row * top + k] = place; tiles: (expert, first place, pairs) for every `tile_m` pairs of an
 // expert; num_tiles[0] = how many.
-__global__ void __launch_bounds__(1024)
-moe_sort_kernel(const int* __restrict__ idx, int pairs, int E, int tile_m, int* __restrict__ offsets,
+// A warp takes a contiguous run of the pairs and counts in a table of its own (`tables` = 32; one for all where that many
+// tables of E numbers do not fit), the lanes that hold the same expert at once; so the pairs of an expert stay in their order and
+// nothing queues at 32 shared counters: 16,384 pairs among 32 experts 24 us, 31 with one atomic a pair.
+constexpr int kSortWarps = 32;
+__global__ void __launch_bounds__(32 * kSortWarps)
+moe_sort_kernel(const int* __restrict__ idx, int pairs, int E, int tile_m, int tables, int* __restrict__ offsets,
                 int* __restrict__ pair_of, int* __restrict__ place_of, int* __restrict__ tile_expert,
                 int* __restrict__ tile_begin, int* __restrict__ tile_rows, int* __restrict__ num_tiles) {
-  extern __shared__ int sort_smem[];
-  int* cnt = sort_smem;
-  int* cursor = sort_smem + E;
-  for (int e = threadIdx.x; e < E; e += blockDim.x) cnt[e] = 0;
+  extern __shared__ int sort_smem[];                       // [tables][E] counts, then next places | [E] first place | [E] first tile
+  pdl_launch_dependents();
+  pdl_wait();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int* first = sort_smem + tables * E;
+  int* first_tile = first + E;
+  int* mine = sort_smem + (tables > 1 ? warp * E : 0);
+  const int run = (pairs + 32 * kSortWarps - 1) / (32 * kSortWarps) * 32;           // pairs of a warp
+  const int begin = warp * run, end = min(pairs, begin + run);
+  for (int i = threadIdx.x; i < tables * E; i += blockDim.x) sort_smem[i] = 0;
   __syncthreads();
-  for (int p = threadIdx.x; p < pairs; p += blockDim.x) atomicAdd(&cnt[idx[p]], 1);
+  // f(pair, expert, lowest lane with this expert, how many lanes before this one hold it, how many at all)
+  auto each = [&](auto f) {
+    constexpr int kAhead = 4;
+    for (int p0 = begin; p0 < end; p0 += 32 * kAhead) {
+      int e[kAhead];
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u) {
+        const int p = p0 + 32 * u + lane;
+        e[u] = p < end ? idx[p] : -1;
+      }
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u) {
+        const unsigned same = __match_any_sync(0xffffffffu, e[u]);
+        f(p0 + 32 * u + lane, e[u], __ffs(same) - 1, __popc(same & ((1u << lane) - 1u)), __popc(same));
+      }
+    }
+  };
+  each([&](int, int e, int leader, int, int count) {
+    if (e >= 0 && lane == leader) atomicAdd(&mine[e], count);
+    __syncwarp();
+  });
+  __syncthreads();
+  for (int e = threadIdx.x; e < E; e += blockDim.x) {      // a table's share of an expert's places; the expert's pairs
+    int at = 0;
+    for (int w = 0; w < tables; ++w) {
+      const int n = sort_smem[w * E + e];
+      sort_smem[w * E + e] = at;
+      at += n;
+    }
+    first[e] = at;
+  }
   __syncthreads();
   if (threadIdx.x == 0) {
     int at = 0, tiles = 0;
     for (int e = 0; e < E; ++e) {
-      offsets[e] = at;
-      cursor[e] = at;
-      for (int b = 0; b < cnt[e]; b += tile_m, ++tiles) {
-        tile_expert[tiles] = e;
-        tile_begin[tiles] = at + b;
-        tile_rows[tiles] = min(tile_m, cnt[e] - b);
-      }
-      at += cnt[e];
+      const int n = first[e];
+      first[e] = at;
+      first_tile[e] = tiles;
+      at += n;
+      tiles += (n + tile_m - 1) / tile_m;
     }
     offsets[E] = at;
     num_tiles[0] = tiles;
   }
   __syncthreads();
-  for (int p = threadIdx.x; p < pairs; p += blockDim.x) {
-    const int place = atomicAdd(&cursor[idx[p]], 1);
-    pair_of[place] = p;
-    place_of[p] = place;
+  for (int e = threadIdx.x; e < E; e += blockDim.x) {
+    offsets[e] = first[e];
+    const int n = (e + 1 < E ? first[e + 1] : pairs) - first[e];
+    for (int b = 0, t = first_tile[e]; b < n; b += tile_m, ++t) {
+      tile_expert[t] = e;
+      tile_begin[t] = first[e] + b;
+      tile_rows[t] = min(tile_m, n - b);
+    }
   }
+  each([&](int p, int e, int leader, int before, int count) {
+    int at = 0;
+    if (e >= 0 && lane == leader) at = atomicAdd(&mine[e], count);
+    at = __shfl_sync(0xffffffffu, at, leader);
+    if (e >= 0) {
+      const int place = first[e] + at + before;
+      pair_of[place] = p;
+      place_of[p] = place;
+    }
+  });
 }
 
 // ----------------------------------------------------------------------------- the products
@@ -706,11 +757,16 @@ inline MoeWork moe_work(int* work, int pairs, int E, int tile_m) {
 }
 
 int launch_moe_sort(const int* idx, int pairs, int E, int tile_m, int* work, cudaStream_t s) {
+  const auto bytes = [&](int tables) { return (size_t(tables) + 2) * E * sizeof(int); };
+  const int tables = bytes(kSortWarps) <= 48 * 1024 ? kSortWarps : 1;
   if (size_t(2 * E) * sizeof(int) > 48 * 1024 || pairs / tile_m + E > 65535) return KVCM_ERR_UNSUPPORTED;
+  if (bytes(tables) > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(moe_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes(tables)));
+    if (e != cudaSuccess) return int(e);
+  }
   const MoeWork w = moe_work(work, pairs, E, tile_m);
-  moe_sort_kernel<<<1, 1024, size_t(2 * E) * sizeof(int), s>>>(idx, pairs, E, tile_m, w.offsets, w.pair_of, w.place_of,
-                                                               w.tile_expert, w.tile_begin, w.tile_rows, w.num_tiles);
-  return KVCM_LAUNCH_RESULT();
+  return pdl_launch(moe_sort_kernel, dim3(1), dim3(32 * kSortWarps), bytes(tables), s, idx, pairs, E, tile_m, tables, w.offsets, w.pair_of,
+                    w.place_of, w.tile_expert, w.tile_begin, w.tile_rows, w.num_tiles);
 }
 
 template <typename T>

@@ -16,6 +16,7 @@
 // behind the end) and drops those results.
 // Every wait on an mbarrier is bounded; when one runs out the block records it
 // (kvcm_moe_tcgen05_error), stops waiting, frees its tensor memory and leaves.
+#include "pdl.cuh"
 #include "tcgen05_common.cuh"
 
 namespace kvcm {
@@ -46,6 +47,7 @@ moe_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
   __shared__ volatile int abort_flag;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  pdl_wait();
   const int n_tiles = (N + BNOUT - 1) / BNOUT;
   const int rows_per_expert = GATED ? 2 * N : N;
   const int tiles = num_tiles[0] * n_tiles;
@@ -72,6 +74,7 @@ moe_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
   __syncthreads();
   tc5::fence_after();
   const uint32_t tmem = tmem_base;
+  pdl_launch_dependents();                       // only with the tensor memory in hand: dependents may take some too
 
   if (warp == 0) {
     if (lane == 0) {
@@ -206,18 +209,31 @@ moe_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
   }
 }
 
-// xs[place] = h[pair_of[place] / top]: the rows of h in the order of the sorted pairs.
+// xs[place] = h[pair_of[place] / top]: the rows of h in the order of the sorted pairs, four of them a block so that four loads
+// are in flight a thread.
+constexpr int kMeGather = 4;
 __global__ void __launch_bounds__(256)
-moe_gather_kernel(const bf16* __restrict__ h, int ldh, const int* __restrict__ pair_of, int top, bf16* __restrict__ xs,
+moe_gather_kernel(const bf16* __restrict__ h, int ldh, const int* __restrict__ pair_of, int pairs, int top, bf16* __restrict__ xs,
                   int D) {
-  const int place = blockIdx.x;
-  const bf16* src = h + size_t(pair_of[place] / top) * ldh;
+  pdl_launch_dependents();
+  pdl_wait();
+  const int place = blockIdx.x * kMeGather, n = min(kMeGather, pairs - place);
+  const bf16* src[kMeGather];
+#pragma unroll
+  for (int u = 0; u < kMeGather; ++u) src[u] = h + size_t(pair_of[place + min(u, n - 1)] / top) * ldh;
   bf16* dst = xs + size_t(place) * D;
   if ((D % 8) == 0 && (ldh % 8) == 0 && (reinterpret_cast<uintptr_t>(h) & 15) == 0) {
-    for (int i = threadIdx.x; i < D / 8; i += blockDim.x)
-      reinterpret_cast<uint4*>(dst)[i] = reinterpret_cast<const uint4*>(src)[i];
+    for (int i = threadIdx.x; i < D / 8; i += blockDim.x) {
+      uint4 v[kMeGather];
+#pragma unroll
+      for (int u = 0; u < kMeGather; ++u) v[u] = reinterpret_cast<const uint4*>(src[u])[i];
+#pragma unroll
+      for (int u = 0; u < kMeGather; ++u)
+        if (u < n) reinterpret_cast<uint4*>(dst + size_t(u) * D)[i] = v[u];
+    }
   } else {
-    for (int i = threadIdx.x; i < D; i += blockDim.x) dst[i] = src[i];
+    for (int u = 0; u < n; ++u)
+      for (int i = threadIdx.x; i < D; i += blockDim.x) dst[size_t(u) * D + i] = src[u][i];
   }
 }
 
@@ -241,9 +257,8 @@ int launch_moe_tcgen05(const void* X, long long x_rows, const void* W, long long
   constexpr int BNOUT = GATED ? kMeBN / 2 : kMeBN;
   const long long most = (long long)max_work_tiles * ((N + BNOUT - 1) / BNOUT);
   const int sms = tc5::current_sm_count();
-  kernel<<<dim3(unsigned(most < sms ? most : sms)), kMeThreads, smem, s>>>(mx, mw, reinterpret_cast<OutT*>(Y), N, K, ldy,
-                                                                         tile_expert, tile_begin, tile_rows, num_tiles);
-  return KVCM_LAUNCH_RESULT();
+  return pdl_launch(kernel, dim3(unsigned(most < sms ? most : sms)), dim3(kMeThreads), smem, s, mx, mw, reinterpret_cast<OutT*>(Y), N, K, ldy,
+                    tile_expert, tile_begin, tile_rows, num_tiles);
 }
 
 }  // namespace kvcm
@@ -266,7 +281,8 @@ KVCM_API int kvcm_moe_experts_tcgen05_bf16(const void* h, int ldh, const void* w
     if (reinterpret_cast<uintptr_t>(p) & 15) return KVCM_ERR_UNSUPPORTED;
   cudaStream_t s = (cudaStream_t)stream;
   const int max_work_tiles = pairs / kMeBM + E;
-  moe_gather_kernel<<<pairs, 256, 0, s>>>((const bf16*)h, ldh, pair_of, top, (bf16*)xs, D);
+  pdl_launch(moe_gather_kernel, dim3((pairs + kMeGather - 1) / kMeGather), dim3(256), 0, s, (const bf16*)h, ldh, pair_of, pairs, top,
+             (bf16*)xs, D);
   int rc = KVCM_LAUNCH_RESULT();
   if (rc) return rc;
   rc = launch_moe_tcgen05<bf16, true>(xs, pairs, wgu, (long long)E * 2 * F, act, F, D, F, tile_expert, tile_begin,

@@ -494,6 +494,32 @@ def test_expert_products_of_few_rows_against_float64(T, E, top, F, D):
     assert torch.allclose(out.double(), (wt.double()[..., None] * y.double().view(T, top, D)).sum(1) + gate.double()[:, None] * shared.double(), atol=1e-5)
 
 
+@pytest.mark.parametrize("T,E,top", [(1, 3, 1), (257, 8, 2), (4100, 5, 4), (70, 361, 3), (70, 362, 3), (33, 6144, 5)])
+def test_sort_of_the_pairs_by_expert(T, E, top):
+    """One table of counts a warp, and (from 362 experts on) one for all: every pair has one place, experts follow one another;
+    with a table a warp the pairs of an expert keep their order."""
+    from kvcm.kernels import library as K
+    g = torch.Generator().manual_seed(T + E)
+    idx = torch.randint(0, E, (T, top), generator=g, dtype=torch.int32).cuda()
+    F = D = 6
+    h, wgu, wd = torch.randn(T, D, device="cuda"), torch.randn(E, 2 * F, D, device="cuda"), torch.randn(E, D, F, device="cuda")
+    work = torch.empty(K.moe_work_ints(T, top, E), dtype=torch.int32, device="cuda")
+    y, out, wt = torch.empty(T * top, D, device="cuda"), torch.empty(T, D, device="cuda"), torch.rand(T, top, device="cuda")
+    K.moe_experts(h, wgu, wd, idx, work, torch.empty(T * top, F, device="cuda"), y)
+    K.moe_combine(y, work, wt, E, None, None, out)
+    n = T * top
+    pair_of, place_of = work[E + 2:E + 2 + n].long(), work[E + 2 + n:E + 2 + 2 * n].long()
+    e = idx.flatten().long()
+    assert torch.equal(pair_of[place_of], torch.arange(n, device="cuda"))
+    assert torch.equal(e[pair_of], e.sort().values)
+    assert torch.equal(work[:E + 1].long(), torch.searchsorted(e.sort().values, torch.arange(E + 1, device="cuda")))
+    if E <= 361:
+        assert torch.equal(pair_of, e.sort(stable=True).indices)
+    # sums of top numbers, each rounded once: top * 2^-24 of their absolute sum
+    parts = wt.double()[..., None] * y[place_of].double().view(T, top, D)
+    assert ((out.double() - parts.sum(1)).abs() <= top * 2.0 ** -23 * parts.abs().sum(1) + 1e-30).all()
+
+
 @pytest.mark.parametrize("T,E,D,gate", [(1, 8, 8, False), (4, 32, 2048, True), (16, 31, 72, False), (17, 39, 2056, True), (64, 60, 520, False)])
 def test_router_split_over_a_cluster_against_float64(T, E, D, gate):
     """Softmax weights and choices of steps of few rows: the logits of both forms are float sums of exact products."""
