@@ -8,7 +8,7 @@
 // with the expert's matrices addressed inside the stacked tensor ([E * rows_per_expert, K]) by a
 // row offset of the tensor-map coordinate.  The kernel is the persistent, warp-specialised one of
 // gemm_tcgen05.cu (TMA ring of 128-byte-swizzled [128 x 64] and [256 x 64] pieces, one thread
-// issuing tcgen05.mma into two accumulators of tensor memory, four epilogue warps reading them
+// issuing tcgen05.mma into two accumulators of tensor memory, eight epilogue warps reading them
 // back with tcgen05.ld) with two changes: the list of work tiles, and how many there are, is
 // read from device memory (nothing about the routing is known on the host, so the step can be
 // recorded into a CUDA graph), and the epilogue stores only the tile's own rows: a tile that holds
@@ -22,7 +22,7 @@
 namespace kvcm {
 
 constexpr int kMeBM = 128, kMeBK = 64, kMeBN = 256;
-constexpr int kMeThreads = 192;
+constexpr int kMeThreads = 320;
 constexpr int kMeABytes = kMeBM * kMeBK * 2;
 constexpr int kMeBBytes = kMeBN * kMeBK * 2;
 constexpr int kMeStageBytes = kMeABytes + kMeBBytes;
@@ -62,7 +62,7 @@ moe_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     }
     for (int a = 0; a < 2; ++a) {
       tc5::mbar_init(&acc_full[a], 1);
-      tc5::mbar_init(&acc_empty[a], 4);                        // four epilogue warps
+      tc5::mbar_init(&acc_empty[a], 8);                        // eight epilogue warps
     }
     tc5::mbar_init_fence();
   }
@@ -137,7 +137,7 @@ moe_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
       }
     }
   } else {
-    const int quarter = warp & 3;
+    const int quarter = warp & 3, half = (warp - 2) >> 2;                // every second 32 columns
     for (int tl = 0; tl < my_tiles; ++tl) {
       const int acc = tl & 1;
       const int t = int(blockIdx.x) + tl * int(gridDim.x);
@@ -152,7 +152,7 @@ moe_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
       const bool row_ok = local < tile_rows[wt];
       const size_t row = size_t(tile_begin[wt]) + local;
 #pragma unroll 1
-      for (int c = 0; c < BNOUT / 32; ++c) {
+      for (int c = half; c < BNOUT / 32; c += 2) {
         const uint32_t taddr = tmem + (uint32_t(quarter * 32) << 16) + uint32_t(acc * kMeBN + c * 32);
         const int col0 = n0 + c * 32;
         if constexpr (GATED) {
