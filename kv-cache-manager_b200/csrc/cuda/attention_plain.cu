@@ -17,7 +17,8 @@
 // What bounds it: the latency of one row's chain of keys (a decode step has few rows), so a key's cache row is looked
 // up once per chunk and kept, elements move four at a time, and the products with V are dealt out over groups of
 // threads that take every n-th key each, joined at the end in the groups' order.  Measured on B200 (float32, 2 requests,
-// 32 heads of 64, 64 to 80 keys): 17.9 us a launch before.
+// 32 heads of 64, 64 to 80 keys): 17.9 us a launch before; eight tokens of two such requests through 22 layers, with the
+// float products' tiles of the same change: 38.4 -> 27.2 ms.
 #include "common.cuh"
 #include "pdl.cuh"
 
