@@ -19,6 +19,7 @@
 // recurrence is one dependent chain per column (dot product, step, update) whose length per token
 // is what bounds a long portion of ONE request; requests and heads run side by side.
 #include "common.cuh"
+#include "pdl.cuh"
 
 namespace kvcm {
 
@@ -34,6 +35,8 @@ delta_conv_kernel(const T* __restrict__ proj, int ldp, const float* __restrict__
                   const int* __restrict__ row_seq, const int* __restrict__ seq_q_start,
                   const int* __restrict__ seq_state_slot, float* __restrict__ out, int channels,
                   const float* __restrict__ bias) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int row = blockIdx.x;
   const int c = blockIdx.y * blockDim.x + threadIdx.x;
   if (c >= channels) return;
@@ -64,6 +67,8 @@ delta_conv_run_kernel(const T* __restrict__ proj, int ldp, const float* __restri
                       const int* __restrict__ row_seq, const int* __restrict__ seq_q_start,
                       const int* __restrict__ seq_state_slot, float* __restrict__ out, int channels, int rows,
                       const float* __restrict__ bias) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int c = blockIdx.y * blockDim.x + threadIdx.x;
   if (c >= channels) return;
   const int r0 = blockIdx.x * kConvRun, r1 = min(rows, r0 + kConvRun);
@@ -125,6 +130,8 @@ __global__ void __launch_bounds__(256)
 delta_conv_state_kernel(const T* __restrict__ proj, int ldp, int taps, float* __restrict__ state,
                         long long state_stride, long long conv_off, const int* __restrict__ seq_q_start,
                         const int* __restrict__ seq_q_len, const int* __restrict__ seq_state_slot, int channels) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int s = blockIdx.x;
   const int c = blockIdx.y * blockDim.x + threadIdx.x;
   const int slot = seq_state_slot[s];
@@ -146,6 +153,8 @@ delta_conv_single_kernel(const T* __restrict__ proj, int ldp, const float* __res
                          float* __restrict__ state, long long state_stride, long long conv_off,
                          const int* __restrict__ seq_q_start, const int* __restrict__ seq_state_slot,
                          float* __restrict__ out, int channels, const float* __restrict__ bias) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int s = blockIdx.x;
   const int c = blockIdx.y * blockDim.x + threadIdx.x;
   if (c >= channels) return;
@@ -171,6 +180,8 @@ delta_conv_single_kernel(const T* __restrict__ proj, int ldp, const float* __res
 __global__ void __launch_bounds__(128)
 delta_prepare_kernel(float* __restrict__ qkv, int channels, float* __restrict__ ba, const float* __restrict__ a_log,
                      const float* __restrict__ dt_bias, int heads, int qk_heads, int dk) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int row = blockIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const float qscale = 1.f / sqrtf(float(dk));
@@ -240,6 +251,8 @@ constexpr int kScanDelta = 0, kScanDeltaChannel = 1, kScanLinear = 2, kScanLinea
 template <int DR_COLS, int DR_LANES, int NI, int TT, bool EARLY, int MODE>
 __global__ void __launch_bounds__(DR_COLS * DR_LANES)
 delta_scan_kernel(const ScanArgs A) {
+  pdl_launch_dependents();
+  pdl_wait();
   const float* __restrict__ qkv = A.qkv;
   const int channels = A.channels, heads = A.heads, qk_heads = A.qk_heads, dk = A.dk, dv = A.dv;
   float* __restrict__ state = A.state;
@@ -495,6 +508,8 @@ template <typename T>
 __global__ void __launch_bounds__(128)
 gated_rms_kernel(const float* __restrict__ o, const T* __restrict__ gate, int ldg, const float* __restrict__ w,
                  T* __restrict__ out, int heads, int dv, float eps) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int row = blockIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   for (int h = blockIdx.y * nwarps + warp; h < heads; h += gridDim.y * nwarps) {
@@ -519,22 +534,19 @@ int launch_delta_conv(const void* proj, int ldp, const float* conv_w, int taps, 
   if (taps < 1) return KVCM_ERR_UNSUPPORTED;
   const int by = (channels + 255) / 256;
   if (rows == seqs) {                            // every request brings one row: rows and requests coincide
-    delta_conv_single_kernel<T><<<dim3(rows, by), 256, 0, s>>>((const T*)proj, ldp, conv_w, taps, state, state_stride, conv_off,
-                                                               seq_q_start, seq_state_slot, out, channels, bias);
-    return KVCM_LAUNCH_RESULT();
+    return pdl_launch(delta_conv_single_kernel<T>, dim3(rows, by), dim3(256), 0, s, (const T*)proj, ldp, conv_w, taps, state,
+                      state_stride, conv_off, seq_q_start, seq_state_slot, out, channels, bias);
   }
   if (taps <= kConvMaxTaps)
-    delta_conv_run_kernel<T><<<dim3((rows + kConvRun - 1) / kConvRun, by), 256, 0, s>>>(
-        (const T*)proj, ldp, conv_w, taps, state, state_stride, conv_off, row_seq, seq_q_start, seq_state_slot, out, channels,
-        rows, bias);
+    pdl_launch(delta_conv_run_kernel<T>, dim3((rows + kConvRun - 1) / kConvRun, by), dim3(256), 0, s, (const T*)proj, ldp, conv_w,
+               taps, state, state_stride, conv_off, row_seq, seq_q_start, seq_state_slot, out, channels, rows, bias);
   else
-    delta_conv_kernel<T><<<dim3(rows, by), 256, 0, s>>>((const T*)proj, ldp, conv_w, taps, state, state_stride, conv_off,
-                                                        row_seq, seq_q_start, seq_state_slot, out, channels, bias);
+    pdl_launch(delta_conv_kernel<T>, dim3(rows, by), dim3(256), 0, s, (const T*)proj, ldp, conv_w, taps, state, state_stride,
+               conv_off, row_seq, seq_q_start, seq_state_slot, out, channels, bias);
   int rc = KVCM_LAUNCH_RESULT();
   if (rc || taps == 1) return rc;
-  delta_conv_state_kernel<T><<<dim3(seqs, by), 256, 0, s>>>((const T*)proj, ldp, taps, state, state_stride, conv_off,
-                                                            seq_q_start, seq_q_len, seq_state_slot, channels);
-  return KVCM_LAUNCH_RESULT();
+  return pdl_launch(delta_conv_state_kernel<T>, dim3(seqs, by), dim3(256), 0, s, (const T*)proj, ldp, taps, state, state_stride,
+                    conv_off, seq_q_start, seq_q_len, seq_state_slot, channels);
 }
 
 }  // namespace kvcm
@@ -560,8 +572,8 @@ KVCM_API int kvcm_delta_prepare(float* qkv, int channels, float* ba, const float
                                 int rows, int heads, int qk_heads, int dk, void* stream) {
   if (rows == 0) return 0;
   const int by = (2 * qk_heads + 3) / 4;                       // a warp per query/key head, four to a block
-  delta_prepare_kernel<<<dim3(rows, by), 128, 0, (cudaStream_t)stream>>>(qkv, channels, ba, a_log, dt_bias, heads, qk_heads, dk);
-  return KVCM_LAUNCH_RESULT();
+  return pdl_launch(delta_prepare_kernel, dim3(rows, by), dim3(128), 0, (cudaStream_t)stream, qkv, channels, ba, a_log, dt_bias,
+                    heads, qk_heads, dk);
 }
 
 // Largest key size the recurrence kernel holds in registers.
@@ -592,7 +604,8 @@ static int launch_scan(const ScanArgs& A, int rows, int seqs, cudaStream_t s) {
   // with a decay per channel a third staged array shares the static shared memory: fewer tokens a tile
   constexpr int TT_LONG = CHD ? 8 : 16, TT_LONGEST = CHD ? 4 : 8;
 #define KVCM_SCAN_E(COLS, LANES, NI, TT, EARLY)                                                                     \
-  delta_scan_kernel<COLS, LANES, NI, TT, EARLY, MODE><<<dim3((dv + COLS - 1) / COLS, heads, seqs), COLS * LANES, 0, s>>>(A)
+  pdl_launch((delta_scan_kernel<COLS, LANES, NI, TT, EARLY, MODE>), dim3((dv + COLS - 1) / COLS, heads, seqs),      \
+             dim3(COLS * LANES), 0, s, A)
 #define KVCM_SCAN_C(COLS, LANES, NI, TT)                                                                            \
   do {                                                                                                              \
     if constexpr (LIN) KVCM_SCAN_E(COLS, LANES, NI, TT, false);                                                     \
@@ -666,6 +679,8 @@ __global__ void __launch_bounds__(128)
 delta_prepare_channel_kernel(float* __restrict__ qkv, int channels, const T* __restrict__ b, int ldb,
                              float* __restrict__ beta, float* __restrict__ a, const float* __restrict__ a_log,
                              const float* __restrict__ dt_bias, int heads, int qk_heads, int dk) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int row = blockIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const float qscale = 1.f / sqrtf(float(dk));
@@ -693,6 +708,8 @@ template <typename T>
 __global__ void __launch_bounds__(128)
 ssm_prepare_kernel(const T* __restrict__ raw, int ld, const float* __restrict__ a_log, const float* __restrict__ dt_bias,
                    float* __restrict__ out, int rows, int heads) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= rows * heads) return;
   const int row = idx / heads, h = idx - row * heads;
@@ -716,6 +733,8 @@ __global__ void __launch_bounds__(128)
 group_rms_gate_kernel(const float* __restrict__ o, const Z* __restrict__ z, int ldz, const float* __restrict__ skip, int lds,
                       const float* __restrict__ skip_coef, int head, const float* __restrict__ w, int wlen,
                       T* __restrict__ out, int n, int group, int gate_first, int act, float eps) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int row = blockIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const int groups = n / group;
@@ -751,6 +770,8 @@ __global__ void __launch_bounds__(256)
 group_rms_gate_wide_kernel(const float* __restrict__ o, const Z* __restrict__ z, int ldz, const float* __restrict__ skip,
                            int lds, const float* __restrict__ skip_coef, int head, const float* __restrict__ w, int wlen,
                            T* __restrict__ out, int n, int group, int gate_first, int act, float eps) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float scratch[33];
   const int row = blockIdx.x, i0 = blockIdx.y * group;
   constexpr int kKeep = 8;                                 // values a thread keeps between the two passes
@@ -805,6 +826,8 @@ template <typename T, typename Z, int NC>      // NC: quads a thread keeps (grou
 __global__ void __launch_bounds__(256)
 group_rms_gate_vec_kernel(const float* __restrict__ o, const Z* __restrict__ z, int ldz, const float* __restrict__ w, int wlen,
                           T* __restrict__ out, int n, int group, int act, float eps) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float scratch[33];
   const int row = blockIdx.x, i0 = blockIdx.y * group;
   float4 v[NC], gz[NC];
@@ -848,21 +871,21 @@ static int launch_group_rms_gate(const float* o, const void* z, int ldz, const f
     const dim3 grid(rows, groups);
     const int need = (group / 4 + 255) / 256;
     if (need <= 2)
-      group_rms_gate_vec_kernel<T, Z, 2><<<grid, 256, 0, s>>>(o, (const Z*)z, ldz, w, wlen, (T*)out, n, group, act, eps);
+      return pdl_launch((group_rms_gate_vec_kernel<T, Z, 2>), grid, dim3(256), 0, s, o, (const Z*)z, ldz, w, wlen, (T*)out, n,
+                        group, act, eps);
     else if (need <= 4)
-      group_rms_gate_vec_kernel<T, Z, 4><<<grid, 256, 0, s>>>(o, (const Z*)z, ldz, w, wlen, (T*)out, n, group, act, eps);
+      return pdl_launch((group_rms_gate_vec_kernel<T, Z, 4>), grid, dim3(256), 0, s, o, (const Z*)z, ldz, w, wlen, (T*)out, n,
+                        group, act, eps);
     else
-      group_rms_gate_vec_kernel<T, Z, 8><<<grid, 256, 0, s>>>(o, (const Z*)z, ldz, w, wlen, (T*)out, n, group, act, eps);
-    return KVCM_LAUNCH_RESULT();
+      return pdl_launch((group_rms_gate_vec_kernel<T, Z, 8>), grid, dim3(256), 0, s, o, (const Z*)z, ldz, w, wlen, (T*)out, n,
+                        group, act, eps);
   }
   if (group > 256 && groups <= 65535) {
-    group_rms_gate_wide_kernel<T, Z><<<dim3(rows, groups), 256, 0, s>>>(o, (const Z*)z, ldz, skip, lds, skip_coef, head, w, wlen,
-                                                                      (T*)out, n, group, gate_first, act, eps);
-    return KVCM_LAUNCH_RESULT();
+    return pdl_launch((group_rms_gate_wide_kernel<T, Z>), dim3(rows, groups), dim3(256), 0, s, o, (const Z*)z, ldz, skip, lds,
+                      skip_coef, head, w, wlen, (T*)out, n, group, gate_first, act, eps);
   }
-  group_rms_gate_kernel<T, Z><<<dim3(rows, (groups + 3) / 4), 128, 0, s>>>(o, (const Z*)z, ldz, skip, lds, skip_coef, head, w, wlen,
-                                                                       (T*)out, n, group, gate_first, act, eps);
-  return KVCM_LAUNCH_RESULT();
+  return pdl_launch((group_rms_gate_kernel<T, Z>), dim3(rows, (groups + 3) / 4), dim3(128), 0, s, o, (const Z*)z, ldz, skip, lds,
+                    skip_coef, head, w, wlen, (T*)out, n, group, gate_first, act, eps);
 }
 
 #define KVCM_GROUP_RMS_ARGS                                                                                          \
@@ -885,45 +908,39 @@ KVCM_API int kvcm_delta_prepare_channel_f32(float* qkv, int channels, const void
                                             const float* a_log, const float* dt_bias, int rows, int heads, int qk_heads,
                                             int dk, void* stream) {
   if (rows == 0) return 0;
-  delta_prepare_channel_kernel<float><<<dim3(rows, max(1, min(16, (heads * dk + 511) / 512))), 128, 0, (cudaStream_t)stream>>>(qkv, channels, (const float*)b, ldb, beta, a,
-                                                                              a_log, dt_bias, heads, qk_heads, dk);
-  return KVCM_LAUNCH_RESULT();
+  return pdl_launch(delta_prepare_channel_kernel<float>, dim3(rows, max(1, min(16, (heads * dk + 511) / 512))), dim3(128), 0,
+                    (cudaStream_t)stream, qkv, channels, (const float*)b, ldb, beta, a, a_log, dt_bias, heads, qk_heads, dk);
 }
 KVCM_API int kvcm_delta_prepare_channel_bf16(float* qkv, int channels, const void* b, int ldb, float* beta, float* a,
                                              const float* a_log, const float* dt_bias, int rows, int heads, int qk_heads,
                                              int dk, void* stream) {
   if (rows == 0) return 0;
-  delta_prepare_channel_kernel<bf16><<<dim3(rows, max(1, min(16, (heads * dk + 511) / 512))), 128, 0, (cudaStream_t)stream>>>(qkv, channels, (const bf16*)b, ldb, beta, a,
-                                                                             a_log, dt_bias, heads, qk_heads, dk);
-  return KVCM_LAUNCH_RESULT();
+  return pdl_launch(delta_prepare_channel_kernel<bf16>, dim3(rows, max(1, min(16, (heads * dk + 511) / 512))), dim3(128), 0,
+                    (cudaStream_t)stream, qkv, channels, (const bf16*)b, ldb, beta, a, a_log, dt_bias, heads, qk_heads, dk);
 }
 
 KVCM_API int kvcm_ssm_prepare_f32(const void* raw, int ld, const float* a_log, const float* dt_bias, float* out, int rows,
                                   int heads, void* stream) {
   if (rows == 0) return 0;
-  ssm_prepare_kernel<float><<<(rows * heads + 127) / 128, 128, 0, (cudaStream_t)stream>>>((const float*)raw, ld, a_log, dt_bias,
-                                                                                         out, rows, heads);
-  return KVCM_LAUNCH_RESULT();
+  return pdl_launch(ssm_prepare_kernel<float>, dim3((rows * heads + 127) / 128), dim3(128), 0, (cudaStream_t)stream, (const
+                    float*)raw, ld, a_log, dt_bias, out, rows, heads);
 }
 KVCM_API int kvcm_ssm_prepare_bf16(const void* raw, int ld, const float* a_log, const float* dt_bias, float* out, int rows,
                                    int heads, void* stream) {
   if (rows == 0) return 0;
-  ssm_prepare_kernel<bf16><<<(rows * heads + 127) / 128, 128, 0, (cudaStream_t)stream>>>((const bf16*)raw, ld, a_log, dt_bias,
-                                                                                        out, rows, heads);
-  return KVCM_LAUNCH_RESULT();
+  return pdl_launch(ssm_prepare_kernel<bf16>, dim3((rows * heads + 127) / 128), dim3(128), 0, (cudaStream_t)stream, (const
+                    bf16*)raw, ld, a_log, dt_bias, out, rows, heads);
 }
 
 KVCM_API int kvcm_gated_rms_f32(const float* o, const void* gate, int ldg, const float* w, void* out, int rows,
                                 int heads, int dv, float eps, void* stream) {
   if (rows == 0) return 0;
-  gated_rms_kernel<float><<<dim3(rows, (heads + 3) / 4), 128, 0, (cudaStream_t)stream>>>(
-      o, (const float*)gate, ldg, w, (float*)out, heads, dv, eps);
-  return KVCM_LAUNCH_RESULT();
+  return pdl_launch(gated_rms_kernel<float>, dim3(rows, (heads + 3) / 4), dim3(128), 0, (cudaStream_t)stream, o, (const
+                    float*)gate, ldg, w, (float*)out, heads, dv, eps);
 }
 KVCM_API int kvcm_gated_rms_bf16(const float* o, const void* gate, int ldg, const float* w, void* out, int rows,
                                  int heads, int dv, float eps, void* stream) {
   if (rows == 0) return 0;
-  gated_rms_kernel<bf16><<<dim3(rows, (heads + 3) / 4), 128, 0, (cudaStream_t)stream>>>(
-      o, (const bf16*)gate, ldg, w, (bf16*)out, heads, dv, eps);
-  return KVCM_LAUNCH_RESULT();
+  return pdl_launch(gated_rms_kernel<bf16>, dim3(rows, (heads + 3) / 4), dim3(128), 0, (cudaStream_t)stream, o, (const bf16*)gate,
+                    ldg, w, (bf16*)out, heads, dv, eps);
 }

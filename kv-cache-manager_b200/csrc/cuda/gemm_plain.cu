@@ -8,6 +8,7 @@
 // * batches of small products (one per head, say) of either type.
 // Single products of float operands (the true 32-bit path) are gemm_f32.cu.
 #include "common.cuh"
+#include "pdl.cuh"
 
 namespace kvcm {
 
@@ -73,6 +74,8 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 gemm_few_rows_kernel(const T* __restrict__ X, const T* __restrict__ W, T* __restrict__ Y, int M, int N, int K,
                      int ldx, int ldw, int ldy, long long bx, long long bw, long long by) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ float xrows[];                 // [M][K]
   X += blockIdx.z * bx;
   W += blockIdx.z * bw;
@@ -130,9 +133,8 @@ template <typename T>
 int launch_gemm_few_rows(const void* X, const void* W, void* Y, int M, int N, int K, int ldx, int ldw, int ldy, int batch,
                          long long bx, long long bw, long long by, cudaStream_t s) {
   const size_t smem = size_t(M) * K * sizeof(float);
-  gemm_few_rows_kernel<T><<<dim3((N + 7) / 8, 1, batch), 256, smem, s>>>((const T*)X, (const T*)W, (T*)Y, M, N, K, ldx, ldw,
-                                                                        ldy, bx, bw, by);
-  return KVCM_LAUNCH_RESULT();
+  return pdl_launch(gemm_few_rows_kernel<T>, dim3((N + 7) / 8, 1, batch), dim3(256), smem, s, (const T*)X, (const T*)W, (T*)Y, M,
+                    N, K, ldx, ldw, ldy, bx, bw, by);
 }
 static bool few_rows(int M, int N, int K, int batch) {
   return M >= 1 && M <= kFewRows && size_t(M) * K * sizeof(float) <= 48 * 1024 && batch >= 1 && batch <= 65535 && N >= 1;

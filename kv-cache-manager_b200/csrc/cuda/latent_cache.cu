@@ -11,6 +11,8 @@ template <typename T>
 __global__ void __launch_bounds__(128)
 latent_norm_cache_kernel(const T* __restrict__ v, int ldv, const float* __restrict__ weight,
                          const int* __restrict__ slot_mapping, T* __restrict__ cache, int width, float eps) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float scratch[33];
   const int row = blockIdx.x;
   const int slot = slot_mapping[row];
@@ -118,16 +120,14 @@ using namespace kvcm;
 KVCM_API int kvcm_latent_norm_cache_f32(const void* v, int ldv, const float* weight, const int* slot_mapping,
                                         void* cache, int rows, int width, float eps, void* stream) {
   if (rows == 0) return 0;
-  latent_norm_cache_kernel<float><<<rows, 128, 0, (cudaStream_t)stream>>>((const float*)v, ldv, weight, slot_mapping,
-                                                                         (float*)cache, width, eps);
-  return KVCM_LAUNCH_RESULT();
+  return pdl_launch(latent_norm_cache_kernel<float>, dim3(rows), dim3(128), 0, (cudaStream_t)stream, (const float*)v, ldv, weight,
+                    slot_mapping, (float*)cache, width, eps);
 }
 KVCM_API int kvcm_latent_norm_cache_bf16(const void* v, int ldv, const float* weight, const int* slot_mapping,
                                          void* cache, int rows, int width, float eps, void* stream) {
   if (rows == 0) return 0;
-  latent_norm_cache_kernel<bf16><<<rows, 128, 0, (cudaStream_t)stream>>>((const bf16*)v, ldv, weight, slot_mapping,
-                                                                        (bf16*)cache, width, eps);
-  return KVCM_LAUNCH_RESULT();
+  return pdl_launch(latent_norm_cache_kernel<bf16>, dim3(rows), dim3(128), 0, (cudaStream_t)stream, (const bf16*)v, ldv, weight,
+                    slot_mapping, (bf16*)cache, width, eps);
 }
 
 #define KVCM_LATENT_ROPE_CACHE_ARGS                                                                                   \

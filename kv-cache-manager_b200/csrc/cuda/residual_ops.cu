@@ -3,6 +3,7 @@
 // Each is instantiated for float (the true 32-bit path) and bfloat16 storage; sums, statistics
 // and the stream itself are always float.
 #include "common.cuh"
+#include "pdl.cuh"
 
 namespace kvcm {
 
@@ -18,6 +19,8 @@ embed_sum_kernel(const int* __restrict__ ids, const int* __restrict__ prev, cons
                  const T* __restrict__ table, const T* __restrict__ pair, const T* __restrict__ place,
                  float* __restrict__ x, T* __restrict__ h, int hidden, int vocab, int buckets,
                  long long mul_prev, long long mul_cur, int max_pos) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int t = blockIdx.x;
   const int id = ids[t];
   const int pos = positions[t];
@@ -48,6 +51,8 @@ template <typename T, typename Y, typename W>
 __global__ void __launch_bounds__(256)
 rms_scale_add_kernel(float* __restrict__ x, const Y* __restrict__ y, const W* __restrict__ weight,
                      T* __restrict__ h, int hidden, float eps, float mult) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float scratch[33];
   extern __shared__ float row_cache[];            // hidden floats: the row of y
   const int r = blockIdx.x;
@@ -88,6 +93,8 @@ template <typename T, typename Y, typename W>
 __global__ void __launch_bounds__(256)
 rms_scale_add_vec_kernel(float* __restrict__ x, const Y* __restrict__ y, const W* __restrict__ weight,
                          T* __restrict__ h, int hidden, float eps, float mult) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float scratch[33];
   extern __shared__ float row_cache[];
   const int r = blockIdx.x;
@@ -113,6 +120,8 @@ rms_scale_add_vec_kernel(float* __restrict__ x, const Y* __restrict__ y, const W
 // out[i] = storage(x[i])
 template <typename T>
 __global__ void cast_rows_kernel(const float* __restrict__ x, T* __restrict__ out, long long n) {
+  pdl_launch_dependents();
+  pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) stf(out + i, x[i]);
 }
@@ -123,9 +132,8 @@ int launch_embed_sum(const int* ids, const int* prev, const int* positions, cons
                      long long mul_prev, long long mul_cur, int max_pos, cudaStream_t s) {
   if (rows == 0) return 0;
   if (pair && (buckets <= 0 || !prev)) return KVCM_ERR_UNSUPPORTED;
-  embed_sum_kernel<T><<<rows, 256, 0, s>>>(ids, prev, positions, (const T*)table, (const T*)pair, (const T*)place, x,
+  return pdl_launch(embed_sum_kernel<T>, dim3(rows), dim3(256), 0, s, ids, prev, positions, (const T*)table, (const T*)pair, (const T*)place, x,
                                            (T*)h, hidden, vocab, buckets, mul_prev, mul_cur, max_pos);
-  return KVCM_LAUNCH_RESULT();
 }
 
 template <typename T>
@@ -140,14 +148,13 @@ int launch_rms_scale_add(float* x, const void* y, int y_f32, const void* w, int 
   do {                                                                                                           \
     auto kernel = vec ? rms_scale_add_vec_kernel<T, Y, W> : rms_scale_add_kernel<T, Y, W>;                       \
     if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);  \
-    kernel<<<rows, 256, smem, s>>>(x, (const Y*)y, (const W*)w, (T*)h, hidden, eps, mult);                       \
+    return pdl_launch(kernel, dim3(rows), dim3(256), smem, s, x, (const Y*)y, (const W*)w, (T*)h, hidden, eps, mult); \
   } while (0)
   if (y_f32 && w_f32) KVCM_RSA(float, float);
   else if (y_f32) KVCM_RSA(float, T);
   else if (w_f32) KVCM_RSA(T, float);
   else KVCM_RSA(T, T);
 #undef KVCM_RSA
-  return KVCM_LAUNCH_RESULT();
 }
 
 }  // namespace kvcm
@@ -168,8 +175,8 @@ using namespace kvcm;
   }                                                                                                               \
   KVCM_API int kvcm_cast_rows_##SUFFIX(const float* x, void* out, long long n, void* stream) {                    \
     if (n == 0) return 0;                                                                                         \
-    cast_rows_kernel<T><<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(x, (T*)out, n);            \
-    return KVCM_LAUNCH_RESULT();                                                                                  \
+    return pdl_launch(cast_rows_kernel<T>, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, (cudaStream_t)stream, x, \
+                      (T*)out, n);                                                                                \
   }
 
 KVCM_RESIDUAL_OPS(f32, float)
