@@ -471,9 +471,10 @@ delta_scan_kernel(const ScanArgs A) {
       return o;
     };
     int t = 0;
-    if constexpr (LIN && !EARLY) {
-      // The linear forms' step does not wait for the read-out: four tokens' read-outs are reduced side by side
-      // (the same sums in the same order as one by one).
+    if constexpr (!EARLY && (LIN || NI <= 16)) {
+      // The state's step does not wait for the read-out: four tokens' read-outs are reduced side by side (the same sums in the
+      // same order as one by one), off the chain from token to token, and a token's k and q are read beside the chain of the one
+      // before.
       for (; t + 4 <= nt; t += 4) {
         float o[4];
 #pragma unroll
@@ -487,6 +488,14 @@ delta_scan_kernel(const ScanArgs A) {
 #pragma unroll
           for (int j = 0; j < 4; ++j) out_col[size_t(t0 + t + j) * out_ld] = o[j];
         }
+      }
+    }
+    if constexpr (EARLY) {                              // two tokens in one body: the second's k and q are read early
+      for (; t + 2 <= nt; t += 2) {
+        const float o0 = token(t, true);
+        if (r == 0 && col_ok) out_col[size_t(t0 + t) * out_ld] = o0;
+        const float o1 = token(t + 1, true);
+        if (r == 0 && col_ok) out_col[size_t(t0 + t + 1) * out_ld] = o1;
       }
     }
 #pragma unroll 1
