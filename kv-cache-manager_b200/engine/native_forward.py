@@ -126,7 +126,8 @@ class NativeForward:
     def takes(self, ctx: StepContext) -> bool:
         o = ctx.options
         return (o.get("native_forward", True) and o.get("gemm", "auto") == "auto"
-                and not any(o.get(k, "auto") != "auto" for k in FORCING_OPTIONS) and ctx.tile_rows == 64)
+                and not any(o.get(k, "auto") != "auto" for k in FORCING_OPTIONS) and ctx.tile_rows == 64
+                and not K.profiling())                           # (a profile wants a mark behind every launch)
 
     def run(self, ctx: StepContext) -> Optional[torch.Tensor]:
         """Float32 logits [wanted rows, vocab] (None when no row is wanted).  Only enqueues device work."""
