@@ -8,8 +8,9 @@
 // thread and few enough registers for four blocks an SM.  A block of the grid's second axis takes the n-th of the chosen
 // experts and looks through the step's choices itself for that expert's pairs, in their order: no sort, no gather, and y
 // lies in the order of the pairs.
-// The down product is launched while the gate/up product runs, and asks for its first weights before the dependency
-// wait: gate/up lets dependents go only after its own wait, so the choices that say which weights are complete by then.
+// Both products read the choices behind their own dependency wait: nothing else makes the router's writes visible to a
+// kernel that was launched early, and a choice is an address here.  (So the down product cannot ask for weights before its
+// wait.)  A choice that names no expert is passed over and reported through the error word of the experts' products.
 // The k index inside a 32-wide block is permuted identically for both operands (thread t of a quad owns k = 8t..8t+7),
 // which makes every load a 16-byte vector.  Partial sums of the warps are added in warp order: reproducible.
 // Measured on B200 (32 experts of 512 x 2,048, a call alone with cold weights): 4 rows of 4 choices, 13 experts hit, 20 us; 8 rows of
@@ -43,14 +44,20 @@ struct FewPick {
   int expert, count;
 };
 
+constexpr int kMfNoExpert = 9;                              // code of a choice that names no expert
+
 // The which-th of the chosen experts (ascending) and its pairs; count 0 where there are no more.  Whole block; ends with a
 // barrier.
-__device__ __forceinline__ void pick_expert(FewPick& s, const int* idx, int pairs, int E, int which) {
+__device__ __forceinline__ void pick_expert(FewPick& s, const int* idx, int pairs, int E, int which, int* error) {
   if (threadIdx.x < 32) {
     const int lane = threadIdx.x;
     s.chosen[lane] = 0u;
     __syncwarp();
-    for (int p = lane; p < pairs; p += 32) atomicOr(&s.chosen[idx[p] >> 5], 1u << (idx[p] & 31));
+    for (int p = lane; p < pairs; p += 32) {
+      const unsigned e = unsigned(idx[p]);
+      if (e < unsigned(E)) atomicOr(&s.chosen[e >> 5], 1u << (e & 31));
+      else if (error != nullptr) atomicExch(error, (kMfNoExpert << 16) | p);
+    }
     __syncwarp();
     const unsigned word = s.chosen[lane];
     int upto = __popc(word);
@@ -77,11 +84,10 @@ __device__ __forceinline__ void pick_expert(FewPick& s, const int* idx, int pair
 }
 
 // acc[j] += 16 matrix rows (this thread: rows g and g + 8 from wa and wb) x the rows x[j] behind columns 8 j.., over the
-// 32-wide blocks of k from kb by `stride` below K (K % 8 == 0; addresses already hold the thread's 8 * t4).  `wait`: the
-// dependency wait comes after the first weights have been asked for.
+// 32-wide blocks of k from kb by `stride` below K (K % 8 == 0; addresses already hold the thread's 8 * t4).
 template <int NT, int AHEAD>
 __device__ __forceinline__ void walk_k(float (&acc)[NT][4], const bf16* wa, const bf16* wb, const bf16* const (&x)[NT], int nt,
-                                       int kb, int stride, int K, int t4, bool wait) {
+                                       int kb, int stride, int K, int t4) {
   const uint4 none = make_uint4(0u, 0u, 0u, 0u);
   for (; kb < K; kb += AHEAD * stride) {
     uint4 a[AHEAD], b[AHEAD];
@@ -92,7 +98,6 @@ __device__ __forceinline__ void walk_k(float (&acc)[NT][4], const bf16* wa, cons
       a[u] = in ? load_stream(wa + k) : none;
       b[u] = in ? load_stream(wb + k) : none;
     }
-    if (wait) { pdl_wait(); wait = false; }
 #pragma unroll
     for (int j = 0; j < NT; ++j) {
       if (j >= nt) break;
@@ -111,16 +116,16 @@ __device__ __forceinline__ void walk_k(float (&acc)[NT][4], const bf16* wa, cons
 template <int NT>
 __global__ void __launch_bounds__(32 * kMfUp, NT == 1 ? 4 : 2)
 moe_few_gate_up_kernel(const bf16* h, int ldh, const bf16* __restrict__ wgu, const int* idx, int pairs, int top, int E, int F, int D,
-                       bf16* act, int* place_of) {
+                       bf16* act, int* place_of, int* error) {
   __shared__ FewPick pick;
   __shared__ __align__(16) float red[kMfUp][16][8 * NT];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
   const int f0 = 8 * blockIdx.x;
+  pdl_launch_dependents();
   pdl_wait();
-  pdl_launch_dependents();                                               // (after the wait: see above)
   if (blockIdx.x == 0 && blockIdx.y == 0)
     for (int i = tid; i < pairs; i += 32 * kMfUp) place_of[i] = i;
-  pick_expert(pick, idx, pairs, E, blockIdx.y);
+  pick_expert(pick, idx, pairs, E, blockIdx.y, error);
   const int n = pick.count;
   const bf16* wa = wgu + (size_t(max(pick.expert, 0)) * 2 * F + f0 + g) * D + 8 * t4;      // (F % 8 == 0: the tile's rows exist)
   for (int n0 = 0; n0 < n; n0 += 8 * NT) {                               // (one trip unless a row chose an expert twice)
@@ -131,7 +136,7 @@ moe_few_gate_up_kernel(const bf16* h, int ldh, const bf16* __restrict__ wgu, con
     float acc[NT][4];
 #pragma unroll
     for (int j = 0; j < NT; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
-    walk_k<NT, kMfUpAhead>(acc, wa, wa + size_t(F) * D, x, (here + 7) / 8, warp * 32, 32 * kMfUp, D, t4, false);
+    walk_k<NT, kMfUpAhead>(acc, wa, wa + size_t(F) * D, x, (here + 7) / 8, warp * 32, 32 * kMfUp, D, t4);
 #pragma unroll
     for (int j = 0; j < NT; ++j) {
       *reinterpret_cast<float2*>(&red[warp][g][8 * j + 2 * t4]) = make_float2(acc[j][0], acc[j][1]);
@@ -157,7 +162,8 @@ moe_few_down_kernel(const bf16* act, const bf16* __restrict__ wd, const int* idx
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
   const int c0 = (blockIdx.x * kMfDown + warp) * 16;
   pdl_launch_dependents();
-  pick_expert(pick, idx, pairs, E, blockIdx.y);
+  pdl_wait();
+  pick_expert(pick, idx, pairs, E, blockIdx.y, nullptr);                 // (gate/up has reported)
   const int n = pick.count;
   if (c0 >= D) return;
   const bf16* wa = wd + (size_t(max(pick.expert, 0)) * D + c0 + g) * F + 8 * t4;           // (D % 8 == 0: rows g exist)
@@ -170,7 +176,7 @@ moe_few_down_kernel(const bf16* act, const bf16* __restrict__ wd, const int* idx
     float acc[NT][4];
 #pragma unroll
     for (int j = 0; j < NT; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
-    walk_k<NT, kMfDownAhead>(acc, wa, wb, x, (here + 7) / 8, 0, 32, F, t4, n0 == 0);
+    walk_k<NT, kMfDownAhead>(acc, wa, wb, x, (here + 7) / 8, 0, 32, F, t4);
 #pragma unroll
     for (int j = 0; j < NT; ++j)
 #pragma unroll
@@ -183,10 +189,10 @@ moe_few_down_kernel(const bf16* act, const bf16* __restrict__ wd, const int* idx
 
 template <int NT>
 int launch_moe_few(const bf16* h, int ldh, const bf16* wgu, const bf16* wd, const int* idx, int pairs, int top, int E, int F, int D,
-                   int* place_of, bf16* act, float* y, cudaStream_t s) {
+                   int* place_of, int* error, bf16* act, float* y, cudaStream_t s) {
   const int most = pairs < E ? pairs : E;                                // as many experts can be chosen
   int rc = pdl_launch(moe_few_gate_up_kernel<NT>, dim3(F / 8, most), dim3(32 * kMfUp), 0, s, h, ldh, wgu, idx, pairs, top, E, F, D, act,
-                      place_of);
+                      place_of, error);
   if (rc) return rc;
   return pdl_launch(moe_few_down_kernel<NT>, dim3((D + 16 * kMfDown - 1) / (16 * kMfDown), most), dim3(32 * kMfDown), 0, s,
                     (const bf16*)act, wd, idx, pairs, E, F, D, y);
@@ -196,12 +202,15 @@ int launch_moe_few(const bf16* h, int ldh, const bf16* wgu, const bf16* wd, cons
 
 using namespace kvcm;
 
+extern "C" const int* kvcm_moe_tcgen05_error_address(void);
+
 KVCM_API int kvcm_moe_few_supports(int rows, int top, int E, int F, int D) {
   return rows >= 1 && rows <= kMfMaxRows && top >= 1 && rows * (long long)top <= kMfMaxPairs && E >= 1 && E <= kMfMaxExperts && F >= 8 &&
          (F % 8) == 0 && D >= 8 && (D % 8) == 0;
 }
 
-// `work`: the scratch of kvcm_moe_work_ints; y [pairs, D] in the order of the pairs.  idx within [0, E).
+// `work`: the scratch of kvcm_moe_work_ints; y [pairs, D] in the order of the pairs; rows of y whose choice
+// is not within [0, E) are left as they are.
 KVCM_API int kvcm_moe_experts_few_bf16(const void* h, int ldh, const void* wgu, const void* wd, const int* idx, int rows, int top, int E,
                                        int F, int D, int* work, void* act, float* y, void* stream) {
   if (rows == 0) return 0;
@@ -212,6 +221,6 @@ KVCM_API int kvcm_moe_experts_few_bf16(const void* h, int ldh, const void* wgu, 
   const int pairs = rows * top;
   int* place_of = work + E + 2 + pairs;                                  // as moe.cu lays it out
   const auto run = rows <= 8 ? launch_moe_few<1> : launch_moe_few<2>;
-  return run((const bf16*)h, ldh, (const bf16*)wgu, (const bf16*)wd, idx, pairs, top, E, F, D, place_of, (bf16*)act, y,
-             (cudaStream_t)stream);
+  return run((const bf16*)h, ldh, (const bf16*)wgu, (const bf16*)wd, idx, pairs, top, E, F, D, place_of,
+             const_cast<int*>(kvcm_moe_tcgen05_error_address()), (bf16*)act, y, (cudaStream_t)stream);
 }

@@ -327,12 +327,15 @@ def attention_plain(q: torch.Tensor, out: torch.Tensor, k_cache: torch.Tensor, v
 # index that the sampling kernels write (csrc/cuda/sampling.cu: status_words).
 STATUS_FAMILIES = ("gemm_stream", "gemm_tcgen05", "gemm_tcgen05_pair", "gemm_tcgen05_splitk", "attention_tcgen05",
                    "moe_tcgen05")
+MOE_NO_EXPERT = 9                       # code of a routed choice outside the experts (csrc/cuda/moe_few.cu)
 
 
 def describe_status(first: int, word: int) -> str:
     """Text for a status pair written by the sampling kernels: ``first`` = 1 + index of the kernel
     family whose error word was set (0 = none), ``word`` = (code << 16) | block."""
     name = STATUS_FAMILIES[first - 1] if 1 <= first <= len(STATUS_FAMILIES) else f"family {first}"
+    if name == "moe_tcgen05" and word >> 16 == MOE_NO_EXPERT:
+        return f"routed experts: choice {word & 0xffff} of a step names no expert; the outputs of this step are not valid"
     return (f"{name}: a bounded wait ran out on the device (code {(word >> 16) & 0xffff}, block {word & 0xffff}); "
             f"the outputs of this step are not valid")
 

@@ -494,6 +494,30 @@ def test_expert_products_of_few_rows_against_float64(T, E, top, F, D):
     assert torch.allclose(out.double(), (wt.double()[..., None] * y.double().view(T, top, D)).sum(1) + gate.double()[:, None] * shared.double(), atol=1e-5)
 
 
+def test_a_choice_that_names_no_expert_is_passed_over_and_reported():
+    """Such a choice adds to no expert's pairs, its row of y stays as it was, and the next check of the error words raises."""
+    from kvcm.kernels import library as K
+    g = torch.Generator().manual_seed(3)
+    T, E, top, F, D = 3, 5, 2, 16, 24
+    h = torch.randn(T, D, generator=g).to(torch.bfloat16).cuda()
+    wgu, wd = (torch.randn(*n, generator=g).to(torch.bfloat16).cuda() for n in ((E, 2 * F, D), (E, D, F)))
+    work = torch.empty(K.moe_work_ints(T, top, E), dtype=torch.int32, device="cuda")
+    ys = []
+    for idx in ([[0, 4], [2, 4], [1, 3]], [[0, 4], [5, 4], [-7, 0x3f8ccccd]]):
+        act = torch.empty(T * top, F, dtype=torch.bfloat16, device="cuda")
+        ys.append(torch.full((T * top, D), -3.0, device="cuda"))
+        K.clear_errors()
+        K.moe_experts_few(h, wgu, wd, torch.tensor(idx, dtype=torch.int32).cuda(), work, act, ys[-1])
+        if not ys[1:]:
+            K.check_errors()
+        else:
+            with pytest.raises(K.KernelError, match="names no expert"):
+                K.check_errors()
+    K.check_errors()                                                  # reported once
+    good = torch.tensor([True, True, False, True, False, False])
+    assert torch.equal(ys[1][good], ys[0][good]) and bool((ys[1][~good] == -3.0).all())
+
+
 @pytest.mark.parametrize("T,E,top", [(1, 3, 1), (257, 8, 2), (4100, 5, 4), (70, 361, 3), (70, 362, 3), (33, 6144, 5)])
 def test_sort_of_the_pairs_by_expert(T, E, top):
     """One table of counts a warp, and (from 362 experts on) one for all: every pair has one place, experts follow one another;
