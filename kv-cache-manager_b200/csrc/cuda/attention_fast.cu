@@ -371,7 +371,7 @@ attn_decode_kernel(DecodeParams p) {
 }
 
 // Merges the partitions of one (request, head): out = sum_p 2^(m_p - M) o_p / sum_p 2^(m_p - M) l_p.
-__global__ void attn_decode_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
+__global__ void attn_decode_merge_kernel(const float* part_o, const float* part_ml,
                                          bf16* __restrict__ out, int out_stride, int nh, int hd, int num_parts,
                                          const float* __restrict__ sink) {
   pdl_launch_dependents();

@@ -49,8 +49,8 @@ template <int VEC> __device__ __forceinline__ void load_n(const bf16* p, float (
 
 template <typename T, int VEC>
 __global__ void __launch_bounds__(kPlainThreads)
-attention_plain_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ out, int out_stride,
-                       const T* __restrict__ k_cache, const T* __restrict__ v_cache,
+attention_plain_kernel(const T* q, int q_stride, T* __restrict__ out, int out_stride,
+                       const T* k_cache, const T* v_cache,
                        const int* __restrict__ block_tables, int max_blocks,
                        const int* __restrict__ row_seq, const int* __restrict__ positions,
                        int nh, int nkv, int hd, int block_size, float scale, int window, float softcap,

@@ -30,8 +30,8 @@ __device__ __forceinline__ float silu_f(float z) { return z / (1.f + expf(-z)); 
 // request when l >= 0, else what the state kept of earlier steps (zeros at the very start).
 template <typename T>
 __global__ void __launch_bounds__(256)
-delta_conv_kernel(const T* __restrict__ proj, int ldp, const float* __restrict__ conv_w, int taps,
-                  const float* __restrict__ state, long long state_stride, long long conv_off,
+delta_conv_kernel(const T* proj, int ldp, const float* __restrict__ conv_w, int taps,
+                  const float* state, long long state_stride, long long conv_off,
                   const int* __restrict__ row_seq, const int* __restrict__ seq_q_start,
                   const int* __restrict__ seq_state_slot, float* __restrict__ out, int channels,
                   const float* __restrict__ bias) {
@@ -62,8 +62,8 @@ delta_conv_kernel(const T* __restrict__ proj, int ldp, const float* __restrict__
 constexpr int kConvMaxTaps = 8, kConvRun = 16;
 template <typename T>
 __global__ void __launch_bounds__(256)
-delta_conv_run_kernel(const T* __restrict__ proj, int ldp, const float* __restrict__ conv_w, int taps,
-                      const float* __restrict__ state, long long state_stride, long long conv_off,
+delta_conv_run_kernel(const T* proj, int ldp, const float* __restrict__ conv_w, int taps,
+                      const float* state, long long state_stride, long long conv_off,
                       const int* __restrict__ row_seq, const int* __restrict__ seq_q_start,
                       const int* __restrict__ seq_state_slot, float* __restrict__ out, int channels, int rows,
                       const float* __restrict__ bias) {
@@ -127,7 +127,7 @@ delta_conv_run_kernel(const T* __restrict__ proj, int ldp, const float* __restri
 // One thread owns one (request, channel) and moves old entries down before it overwrites them.
 template <typename T>
 __global__ void __launch_bounds__(256)
-delta_conv_state_kernel(const T* __restrict__ proj, int ldp, int taps, float* __restrict__ state,
+delta_conv_state_kernel(const T* proj, int ldp, int taps, float* state,
                         long long state_stride, long long conv_off, const int* __restrict__ seq_q_start,
                         const int* __restrict__ seq_q_len, const int* __restrict__ seq_state_slot, int channels) {
   pdl_launch_dependents();
@@ -149,8 +149,8 @@ delta_conv_state_kernel(const T* __restrict__ proj, int ldp, int taps, float* __
 // (request, channel), reads the kept inputs, writes the output and moves the state on.
 template <typename T>
 __global__ void __launch_bounds__(256)
-delta_conv_single_kernel(const T* __restrict__ proj, int ldp, const float* __restrict__ conv_w, int taps,
-                         float* __restrict__ state, long long state_stride, long long conv_off,
+delta_conv_single_kernel(const T* proj, int ldp, const float* __restrict__ conv_w, int taps,
+                         float* state, long long state_stride, long long conv_off,
                          const int* __restrict__ seq_q_start, const int* __restrict__ seq_state_slot,
                          float* __restrict__ out, int channels, const float* __restrict__ bias) {
   pdl_launch_dependents();
@@ -178,7 +178,7 @@ delta_conv_single_kernel(const T* __restrict__ proj, int ldp, const float* __res
 // qkv[row]: the first 2 * qk_heads heads of dk (queries, then keys) become unit vectors
 // (x / sqrt(sum x^2 + 1e-6); queries also times dk^-1/2).  ba[row] = [b | a] becomes [beta | g].
 __global__ void __launch_bounds__(128)
-delta_prepare_kernel(float* __restrict__ qkv, int channels, float* __restrict__ ba, const float* __restrict__ a_log,
+delta_prepare_kernel(float* qkv, int channels, float* ba, const float* __restrict__ a_log,
                      const float* __restrict__ dt_bias, int heads, int qk_heads, int dk) {
   pdl_launch_dependents();
   pdl_wait();
@@ -253,9 +253,9 @@ __global__ void __launch_bounds__(DR_COLS * DR_LANES)
 delta_scan_kernel(const ScanArgs A) {
   pdl_launch_dependents();
   pdl_wait();
-  const float* __restrict__ qkv = A.qkv;
+  const float* qkv = A.qkv;
   const int channels = A.channels, heads = A.heads, qk_heads = A.qk_heads, dk = A.dk, dv = A.dv;
-  float* __restrict__ state = A.state;
+  float* state = A.state;
   const long long state_stride = A.state_stride;
   const int* __restrict__ seq_q_start = A.seq_q_start;
   const int* __restrict__ seq_q_len = A.seq_q_len;
@@ -515,7 +515,7 @@ delta_scan_kernel(const ScanArgs A) {
 // out[row, h, j] = storage( o[row, h, j] / sqrt(mean_j o^2 + eps) * w[j] * silu(gate[row, h, j]) )
 template <typename T>
 __global__ void __launch_bounds__(128)
-gated_rms_kernel(const float* __restrict__ o, const T* __restrict__ gate, int ldg, const float* __restrict__ w,
+gated_rms_kernel(const float* o, const T* gate, int ldg, const float* __restrict__ w,
                  T* __restrict__ out, int heads, int dv, float eps) {
   pdl_launch_dependents();
   pdl_wait();
@@ -685,8 +685,8 @@ KVCM_API int kvcm_delta_scan(const float* qkv, int channels, const float* bg, fl
 // a[row, h, i] (float, in place) becomes the decay exp(-exp(A_log[h]) softplus(a + dt_bias[h, i])).
 template <typename T>
 __global__ void __launch_bounds__(128)
-delta_prepare_channel_kernel(float* __restrict__ qkv, int channels, const T* __restrict__ b, int ldb,
-                             float* __restrict__ beta, float* __restrict__ a, const float* __restrict__ a_log,
+delta_prepare_channel_kernel(float* qkv, int channels, const T* b, int ldb,
+                             float* __restrict__ beta, float* a, const float* __restrict__ a_log,
                              const float* __restrict__ dt_bias, int heads, int qk_heads, int dk) {
   pdl_launch_dependents();
   pdl_wait();
@@ -715,7 +715,7 @@ delta_prepare_channel_kernel(float* __restrict__ qkv, int channels, const T* __r
 // decay = exp(-exp(A_log) dt); out rows are [dt | decay].
 template <typename T>
 __global__ void __launch_bounds__(128)
-ssm_prepare_kernel(const T* __restrict__ raw, int ld, const float* __restrict__ a_log, const float* __restrict__ dt_bias,
+ssm_prepare_kernel(const T* raw, int ld, const float* __restrict__ a_log, const float* __restrict__ dt_bias,
                    float* __restrict__ out, int rows, int heads) {
   pdl_launch_dependents();
   pdl_wait();
@@ -739,7 +739,7 @@ __device__ __forceinline__ float gate_act(float z, int act) {
 }
 template <typename T, typename Z>
 __global__ void __launch_bounds__(128)
-group_rms_gate_kernel(const float* __restrict__ o, const Z* __restrict__ z, int ldz, const float* __restrict__ skip, int lds,
+group_rms_gate_kernel(const float* o, const Z* z, int ldz, const float* skip, int lds,
                       const float* __restrict__ skip_coef, int head, const float* __restrict__ w, int wlen,
                       T* __restrict__ out, int n, int group, int gate_first, int act, float eps) {
   pdl_launch_dependents();
@@ -776,7 +776,7 @@ group_rms_gate_kernel(const float* __restrict__ o, const Z* __restrict__ z, int 
 // loads are in flight together instead of one warp walking it.
 template <typename T, typename Z>
 __global__ void __launch_bounds__(256)
-group_rms_gate_wide_kernel(const float* __restrict__ o, const Z* __restrict__ z, int ldz, const float* __restrict__ skip,
+group_rms_gate_wide_kernel(const float* o, const Z* z, int ldz, const float* skip,
                            int lds, const float* __restrict__ skip_coef, int head, const float* __restrict__ w, int wlen,
                            T* __restrict__ out, int n, int group, int gate_first, int act, float eps) {
   pdl_launch_dependents();
@@ -833,7 +833,7 @@ __device__ __forceinline__ void rms_store4(bf16* p, float4 v) {
 }
 template <typename T, typename Z, int NC>      // NC: quads a thread keeps (group <= 256 * 4 * NC)
 __global__ void __launch_bounds__(256)
-group_rms_gate_vec_kernel(const float* __restrict__ o, const Z* __restrict__ z, int ldz, const float* __restrict__ w, int wlen,
+group_rms_gate_vec_kernel(const float* o, const Z* z, int ldz, const float* __restrict__ w, int wlen,
                           T* __restrict__ out, int n, int group, int act, float eps) {
   pdl_launch_dependents();
   pdl_wait();

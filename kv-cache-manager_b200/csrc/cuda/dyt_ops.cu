@@ -15,8 +15,8 @@ namespace kvcm {
 
 template <typename T>
 __global__ void __launch_bounds__(256)
-dyt_norm_kernel(float* __restrict__ x, const float* __restrict__ p0, float s0, const float* __restrict__ p1, float s1,
-                const float* __restrict__ p2, float s2, const float* __restrict__ w, const float* __restrict__ b,
+dyt_norm_kernel(float* x, const float* p0, float s0, const float* p1, float s1,
+                const float* p2, float s2, const float* __restrict__ w, const float* __restrict__ b,
                 const float* __restrict__ alpha, T* __restrict__ out, const int* __restrict__ rows, int hidden) {
   pdl_launch_dependents();
   pdl_wait();
@@ -42,8 +42,8 @@ dyt_norm_kernel(float* __restrict__ x, const float* __restrict__ p0, float s0, c
 // Four elements a thread (hidden % 4 == 0; every row then starts on a 16-byte boundary).
 template <typename T>
 __global__ void __launch_bounds__(256)
-dyt_norm_vec_kernel(float* __restrict__ x, const float* __restrict__ p0, float s0, const float* __restrict__ p1, float s1,
-                    const float* __restrict__ p2, float s2, const float* __restrict__ w, const float* __restrict__ b,
+dyt_norm_vec_kernel(float* x, const float* p0, float s0, const float* p1, float s1,
+                    const float* p2, float s2, const float* __restrict__ w, const float* __restrict__ b,
                     const float* __restrict__ alpha, T* __restrict__ out, const int* __restrict__ rows, int hidden) {
   pdl_launch_dependents();
   pdl_wait();

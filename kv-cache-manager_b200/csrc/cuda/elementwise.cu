@@ -67,7 +67,7 @@ __global__ void embed_vec_kernel(const int* __restrict__ ids, const T* __restric
 // written back to x then.  The weight may be float or T (a tensor stored in 32 bits stays so).
 template <typename T, typename W>
 __global__ void __launch_bounds__(256)
-rmsnorm_kernel(float* __restrict__ x, const T* __restrict__ delta, const W* __restrict__ weight,
+rmsnorm_kernel(float* x, const T* delta, const W* __restrict__ weight,
                T* __restrict__ out, const int* __restrict__ rows, int hidden, float eps) {
   __shared__ float scratch[33];
   extern __shared__ float row_cache[];            // hidden floats: the (updated) row
@@ -100,7 +100,7 @@ rmsnorm_kernel(float* __restrict__ x, const T* __restrict__ delta, const W* __re
 // registers, one pass over global memory, four elements an access.
 template <typename T, typename W, int VEC>
 __global__ void __launch_bounds__(256)
-rmsnorm_vec_kernel(float* __restrict__ x, const T* __restrict__ delta, const W* __restrict__ weight,
+rmsnorm_vec_kernel(float* x, const T* delta, const W* __restrict__ weight,
                    T* __restrict__ out, const int* __restrict__ rows, int hidden, float eps) {
   __shared__ float scratch[33];
   pdl_launch_dependents();
@@ -109,17 +109,23 @@ rmsnorm_vec_kernel(float* __restrict__ x, const T* __restrict__ delta, const W* 
   const int src = rows ? rows[r] : r;
   float* xr = x + size_t(src) * hidden;
   const T* dr = delta ? delta + size_t(src) * hidden : nullptr;
-  float4 v[VEC];
+  float4 v[VEC], d[VEC];
   float ss = 0.f;
+#pragma unroll
+  for (int k = 0; k < VEC; ++k) {                 // (all of the row is asked for before the first store)
+    const int i = (k * 256 + threadIdx.x) * 4;
+    v[k] = d[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (i < hidden) {
+      v[k] = *reinterpret_cast<const float4*>(xr + i);
+      if (dr) d[k] = load4(dr + i);
+    }
+  }
 #pragma unroll
   for (int k = 0; k < VEC; ++k) {
     const int i = (k * 256 + threadIdx.x) * 4;
-    v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (i < hidden) {
-      v[k] = *reinterpret_cast<const float4*>(xr + i);
       if (dr) {
-        const float4 d = load4(dr + i);
-        v[k].x += d.x; v[k].y += d.y; v[k].z += d.z; v[k].w += d.w;
+        v[k].x += d[k].x; v[k].y += d[k].y; v[k].z += d[k].z; v[k].w += d[k].w;
         if (!rows) *reinterpret_cast<float4*>(xr + i) = v[k];
       }
       ss += v[k].x * v[k].x + v[k].y * v[k].y + v[k].z * v[k].z + v[k].w * v[k].w;
@@ -155,7 +161,7 @@ __global__ void add_residual_kernel(float* __restrict__ x, const T* __restrict__
 // slot < 0: the row writes nothing (padding).  write_cache = 0: only the q heads are rotated.
 template <typename T>
 __global__ void __launch_bounds__(256)
-rope_cache_kernel(T* __restrict__ qkv, int row_stride, const int* __restrict__ positions,
+rope_cache_kernel(T* qkv, int row_stride, const int* __restrict__ positions,
                   const float* __restrict__ inv_freq, int rotary_dim, int interleaved,
                   const int* __restrict__ slot_mapping, T* __restrict__ k_cache,
                   T* __restrict__ v_cache, int nh, int nkv, int hd, int block_size,
@@ -204,7 +210,7 @@ rope_cache_kernel(T* __restrict__ qkv, int row_stride, const int* __restrict__ p
 // pairs of a head, i.e. one 16-byte piece of each half, so every access to qkv and to the cache
 // page is a 16-byte vector.  One block per row; the same values as the kernel above.
 __global__ void __launch_bounds__(256)
-rope_cache_vec_kernel(bf16* __restrict__ qkv, int row_stride, const int* __restrict__ positions,
+rope_cache_vec_kernel(bf16* qkv, int row_stride, const int* __restrict__ positions,
                       const float* __restrict__ inv_freq, const int* __restrict__ slot_mapping,
                       bf16* __restrict__ k_cache, bf16* __restrict__ v_cache, int nh, int nkv, int hd,
                       int block_size, int write_cache) {
@@ -267,7 +273,7 @@ __global__ void rope_table_kernel(const int* __restrict__ positions, const float
 // rope_cache_vec_kernel with the angles from that table: no shared memory, no barrier, one item (8
 // neighbouring pairs of a head of a row) a thread.
 __global__ void __launch_bounds__(256)
-rope_cache_table_kernel(bf16* __restrict__ qkv, int row_stride, const float* __restrict__ table,
+rope_cache_table_kernel(bf16* qkv, int row_stride, const float* table,
                         const int* __restrict__ slot_mapping, bf16* __restrict__ k_cache, bf16* __restrict__ v_cache,
                         int rows, int nh, int nkv, int hd, int block_size, int write_cache) {
   pdl_launch_dependents();
@@ -316,7 +322,7 @@ rope_cache_table_kernel(bf16* __restrict__ qkv, int row_stride, const float* __r
 // gate = columns [0, I) of the fused product, up = columns [I, 2I) (activations: gated_act.cuh; SiLU is rounded
 // to the storage type before the product, src/cuda/kernels.cu:72-82).
 template <typename T, int KIND>
-__global__ void gated_act_kernel(const T* __restrict__ gate_up, T* __restrict__ out, int inter, GatedAct act) {
+__global__ void gated_act_kernel(const T* gate_up, T* __restrict__ out, int inter, GatedAct act) {
   pdl_launch_dependents();
   pdl_wait();
   const int t = blockIdx.x;
@@ -328,7 +334,7 @@ __global__ void gated_act_kernel(const T* __restrict__ gate_up, T* __restrict__ 
 
 // bfloat16, width a multiple of 8: eight elements per thread through 16-byte loads and stores.
 template <int KIND>
-__global__ void gated_act_vec_kernel(const bf16* __restrict__ gate_up, bf16* __restrict__ out, int inter, GatedAct act) {
+__global__ void gated_act_vec_kernel(const bf16* gate_up, bf16* __restrict__ out, int inter, GatedAct act) {
   pdl_launch_dependents();
   pdl_wait();
   const int t = blockIdx.x;

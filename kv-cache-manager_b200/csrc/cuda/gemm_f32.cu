@@ -55,7 +55,7 @@ struct F32Tile {
 
 template <typename C, bool VEC>
 __global__ void __launch_bounds__(C::THREADS)
-gemm_f32_kernel(const float* __restrict__ X, const float* __restrict__ W, float* __restrict__ Y, int M, int N, int K,
+gemm_f32_kernel(const float* X, const float* __restrict__ W, float* __restrict__ Y, int M, int N, int K,
                 int ldx, int ldw, int ldy, int S, int seg, int mtiles, int weights_ready) {
   extern __shared__ __align__(16) float f32_smem[];
   constexpr int BM = C::BM, BN = C::BN, TM = C::TM, TN = C::TN, STAGES = C::STAGES;

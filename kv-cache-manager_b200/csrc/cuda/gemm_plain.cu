@@ -72,7 +72,7 @@ constexpr int kFewRows = 16;
 
 template <typename T>
 __global__ void __launch_bounds__(256)
-gemm_few_rows_kernel(const T* __restrict__ X, const T* __restrict__ W, T* __restrict__ Y, int M, int N, int K,
+gemm_few_rows_kernel(const T* X, const T* W, T* __restrict__ Y, int M, int N, int K,
                      int ldx, int ldw, int ldy, long long bx, long long bw, long long by) {
   pdl_launch_dependents();
   pdl_wait();

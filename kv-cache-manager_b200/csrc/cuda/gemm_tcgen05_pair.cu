@@ -153,7 +153,7 @@ template <typename OutT, bool GATED, bool WIDE>
 __global__ void __launch_bounds__(kPairThreads, 1)
 gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                          OutT* __restrict__ Y, int M, int N, int K, int ldy, int BN, int band_rows,
-                         float* __restrict__ part, int* __restrict__ part_flag) {
+                         float* part, int* part_flag) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   __shared__ __align__(8) uint64_t full[kPairStages], empty[kPairStages], acc_full[2], acc_empty[2];

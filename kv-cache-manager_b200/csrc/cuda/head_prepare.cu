@@ -367,7 +367,7 @@ head_prepare_any_kernel(const __grid_constant__ HeadPrepareParams p) {
 // Behind the convolution: the state keeps the last taps - 1 inputs of every request.  One thread owns one (request, channel)
 // and moves old entries down before it overwrites them.
 __global__ void __launch_bounds__(256)
-head_conv_state_kernel(const float* __restrict__ cols, long long ldp, int taps, float* __restrict__ state, long long state_stride,
+head_conv_state_kernel(const float* cols, long long ldp, int taps, float* state, long long state_stride,
                        const int* __restrict__ seq_q_start, const int* __restrict__ seq_q_len,
                        const int* __restrict__ seq_state_slot, int channels) {
   pdl_launch_dependents();

@@ -191,7 +191,7 @@ template <> struct Quad<bf16> {
 
 template <typename T, int PER>
 __global__ void __launch_bounds__(256)
-diff_combine_kernel(const T* __restrict__ a, const float* __restrict__ gate, int ldg, const float* __restrict__ lambda,
+diff_combine_kernel(const T* a, const float* gate, int ldg, const float* __restrict__ lambda,
                     T* __restrict__ out, int rows, int H, int dv, int HD, float eps, float post) {
   pdl_launch_dependents();
   const float lam = lambda[0];
@@ -240,7 +240,7 @@ diff_combine_kernel(const T* __restrict__ a, const float* __restrict__ gate, int
 // heads of HD elements of which the first dv count (HD == dv: plain rows); gate and out have them side by side.
 template <typename T, int V>
 __global__ void __launch_bounds__(256)
-gate_mul_kernel(const T* __restrict__ x, const float* __restrict__ gate, int ldg, T* __restrict__ out, int n, int dv, int HD) {
+gate_mul_kernel(const T* x, const float* gate, int ldg, T* __restrict__ out, int n, int dv, int HD) {
   pdl_launch_dependents();
   pdl_wait();
   const int row = blockIdx.x;

@@ -9,7 +9,7 @@ namespace kvcm {
 
 template <typename T>
 __global__ void __launch_bounds__(128)
-latent_norm_cache_kernel(const T* __restrict__ v, int ldv, const float* __restrict__ weight,
+latent_norm_cache_kernel(const T* v, int ldv, const float* __restrict__ weight,
                          const int* __restrict__ slot_mapping, T* __restrict__ cache, int width, float eps) {
   pdl_launch_dependents();
   pdl_wait();
@@ -37,7 +37,7 @@ latent_norm_cache_kernel(const T* __restrict__ v, int ldv, const float* __restri
 // (2i, 2i+1) (`interleaved`) or (i, i + rot/2); it is not normalised.  Statistics, angles and the turn in float.
 template <typename T>
 __global__ void __launch_bounds__(128)
-latent_rope_cache_kernel(const float* __restrict__ proj, int ldp, const float* __restrict__ wq, const float* __restrict__ wc,
+latent_rope_cache_kernel(const float* proj, int ldp, const float* __restrict__ wq, const float* __restrict__ wc,
                          const int* __restrict__ positions, const float* __restrict__ inv_freq, int rot, int interleaved,
                          const int* __restrict__ slot_mapping, T* __restrict__ cq_out, T* __restrict__ cache, int qr, int R,
                          int dr, int HD, float eps) {
@@ -84,7 +84,7 @@ latent_rope_cache_kernel(const float* __restrict__ proj, int ldp, const float* _
 // (qrow[row, head, 0 : R] is written by that map.)
 template <typename T>
 __global__ void __launch_bounds__(128)
-latent_q_rope_kernel(const float* __restrict__ q, int ldq, const int* __restrict__ positions,
+latent_q_rope_kernel(const float* q, int ldq, const int* __restrict__ positions,
                      const float* __restrict__ inv_freq, int rot, int interleaved, T* __restrict__ qn_out,
                      T* __restrict__ qrow, int H, int dn, int dr, int R, int HD) {
   extern __shared__ __align__(16) float cs_table[];      // rot/2 cosines, rot/2 sines

@@ -293,7 +293,7 @@ __device__ __forceinline__ void route_mma(float (&d)[4], uint32_t a0, uint32_t a
 
 template <int NT>                                           // 8 * NT experts at a time
 __global__ void __launch_bounds__(ROUTE_WARPS * 32)
-moe_route_mma_kernel(const bf16* __restrict__ h, int ldh, const bf16* __restrict__ wr, int rows, int D, RouteChoice choice) {
+moe_route_mma_kernel(const bf16* h, int ldh, const bf16* __restrict__ wr, int rows, int D, RouteChoice choice) {
   constexpr int NP = 8 * NT;
   extern __shared__ float route_smem[];
   pdl_launch_dependents();
@@ -437,7 +437,7 @@ moe_route_few_kernel(const bf16* h, int ldh, const bf16* __restrict__ wr, int ro
 // nothing queues at 32 shared counters: 16,384 pairs among 32 experts 24 us, 31 with one atomic a pair.
 constexpr int kSortWarps = 32;
 __global__ void __launch_bounds__(32 * kSortWarps)
-moe_sort_kernel(const int* __restrict__ idx, int pairs, int E, int tile_m, int tables, int* __restrict__ offsets,
+moe_sort_kernel(const int* idx, int pairs, int E, int tile_m, int tables, int* __restrict__ offsets,
                 int* __restrict__ pair_of, int* __restrict__ place_of, int* __restrict__ tile_expert,
                 int* __restrict__ tile_begin, int* __restrict__ tile_rows, int* __restrict__ num_tiles) {
   extern __shared__ int sort_smem[];                       // [tables][E] counts, then next places | [E] first place | [E] first tile
@@ -643,8 +643,8 @@ moe_down_kernel(const T* __restrict__ act, const T* __restrict__ wd, const int* 
 constexpr int kCombineAhead = 8;
 template <bool VEC>
 __global__ void __launch_bounds__(256)
-moe_combine_kernel(const float* __restrict__ y, const int* __restrict__ place_of, const float* __restrict__ wt, int top,
-                   const float* __restrict__ shared_y, const float* __restrict__ gate, float* __restrict__ out, int D) {
+moe_combine_kernel(const float* y, const int* place_of, const float* wt, int top,
+                   const float* shared_y, const float* gate, float* __restrict__ out, int D) {
   pdl_launch_dependents();
   pdl_wait();
   const int row = blockIdx.x;

@@ -36,9 +36,9 @@ __device__ int g_moe_tcgen05_error = 0;
 template <typename OutT, bool GATED>
 __global__ void __launch_bounds__(kMeThreads)
 moe_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
-                   OutT* __restrict__ Y, int N, int K, int ldy, const int* __restrict__ tile_expert,
-                   const int* __restrict__ tile_begin, const int* __restrict__ tile_rows,
-                   const int* __restrict__ num_tiles) {
+                   OutT* __restrict__ Y, int N, int K, int ldy, const int* tile_expert,
+                   const int* tile_begin, const int* tile_rows,
+                   const int* num_tiles) {
   constexpr int BNOUT = GATED ? kMeBN / 2 : kMeBN;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -213,7 +213,7 @@ moe_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
 // are in flight a thread.
 constexpr int kMeGather = 4;
 __global__ void __launch_bounds__(256)
-moe_gather_kernel(const bf16* __restrict__ h, int ldh, const int* __restrict__ pair_of, int pairs, int top, bf16* __restrict__ xs,
+moe_gather_kernel(const bf16* h, int ldh, const int* pair_of, int pairs, int top, bf16* __restrict__ xs,
                   int D) {
   pdl_launch_dependents();
   pdl_wait();

@@ -49,7 +49,7 @@ embed_sum_kernel(const int* __restrict__ ids, const int* __restrict__ prev, cons
 // y may be float or the storage type; the weight float or the storage type.
 template <typename T, typename Y, typename W>
 __global__ void __launch_bounds__(256)
-rms_scale_add_kernel(float* __restrict__ x, const Y* __restrict__ y, const W* __restrict__ weight,
+rms_scale_add_kernel(float* x, const Y* y, const W* __restrict__ weight,
                      T* __restrict__ h, int hidden, float eps, float mult) {
   pdl_launch_dependents();
   pdl_wait();
@@ -91,7 +91,7 @@ __device__ __forceinline__ void ro_store4(bf16* p, float4 v) {
 
 template <typename T, typename Y, typename W>
 __global__ void __launch_bounds__(256)
-rms_scale_add_vec_kernel(float* __restrict__ x, const Y* __restrict__ y, const W* __restrict__ weight,
+rms_scale_add_vec_kernel(float* x, const Y* y, const W* __restrict__ weight,
                          T* __restrict__ h, int hidden, float eps, float mult) {
   pdl_launch_dependents();
   pdl_wait();
@@ -119,7 +119,7 @@ rms_scale_add_vec_kernel(float* __restrict__ x, const Y* __restrict__ y, const W
 
 // out[i] = storage(x[i])
 template <typename T>
-__global__ void cast_rows_kernel(const float* __restrict__ x, T* __restrict__ out, long long n) {
+__global__ void cast_rows_kernel(const float* x, T* __restrict__ out, long long n) {
   pdl_launch_dependents();
   pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;

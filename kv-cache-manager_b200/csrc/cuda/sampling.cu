@@ -49,7 +49,7 @@ __device__ __forceinline__ void argmax_merge(float& bv, int& bi, float ov, int o
 }
 
 // Block-wide argmax of a row; every thread returns the same (value, index).
-__device__ void block_argmax(const float* __restrict__ row, int vocab, float& best, int& index,
+__device__ void block_argmax(const float* row, int vocab, float& best, int& index,
                              float* sv, int* si) {
   float bv = -INFINITY;
   int bi = 0x7fffffff;
@@ -101,7 +101,7 @@ __device__ void block_argmax(const float* __restrict__ row, int vocab, float& be
 }
 
 __global__ void __launch_bounds__(kSampleThreads)
-argmax_kernel(const float* __restrict__ logits, int* __restrict__ out, int vocab, StatusWords sw, int* status,
+argmax_kernel(const float* logits, int* __restrict__ out, int vocab, StatusWords sw, int* status,
               int* mirror) {
   __shared__ float sv[32];
   __shared__ int si[32];
@@ -128,7 +128,7 @@ __device__ __forceinline__ float sampling_uniform(unsigned long long seed, long 
 }
 
 __global__ void __launch_bounds__(kSampleThreads)
-sample_kernel(const float* __restrict__ logits, const float* __restrict__ temperature,
+sample_kernel(const float* logits, const float* __restrict__ temperature,
               const unsigned long long* __restrict__ seed, const long long* __restrict__ request_id,
               const int* __restrict__ position, int* __restrict__ out, int vocab, StatusWords sw, int* status, int* mirror) {
   __shared__ float sv[32];

@@ -281,7 +281,7 @@ norm_post_pre_regs_kernel(NormPostPreParams p) {
 
 template <typename T>
 __global__ void __launch_bounds__(256)
-poly_norm_act_kernel(const float* __restrict__ z, int ldz, const float* __restrict__ coef, T* __restrict__ out, int F,
+poly_norm_act_kernel(const float* z, int ldz, const float* __restrict__ coef, T* __restrict__ out, int F,
                      float eps) {
   extern __shared__ __align__(16) float row[];
   __shared__ float scratch[33];
@@ -312,7 +312,7 @@ poly_norm_act_kernel(const float* __restrict__ z, int ldz, const float* __restri
 
 template <typename T>
 __global__ void __launch_bounds__(512)
-poly_norm_act_vec_kernel(const float* __restrict__ z, int ldz, const float* __restrict__ coef, T* __restrict__ out, int F,
+poly_norm_act_vec_kernel(const float* z, int ldz, const float* __restrict__ coef, T* __restrict__ out, int F,
                          float eps) {
   extern __shared__ __align__(16) float row[];
   __shared__ float scratch[33];
@@ -349,7 +349,7 @@ poly_norm_act_vec_kernel(const float* __restrict__ z, int ldz, const float* __re
 
 template <typename T>
 __global__ void __launch_bounds__(256)
-concat_cast_kernel(const float* __restrict__ a, const float* __restrict__ b, T* __restrict__ out, int H) {
+concat_cast_kernel(const float* a, const float* b, T* __restrict__ out, int H) {
   pdl_launch_dependents();
   pdl_wait();
   const size_t t = blockIdx.x;
@@ -360,7 +360,7 @@ concat_cast_kernel(const float* __restrict__ a, const float* __restrict__ b, T* 
 }
 
 __global__ void __launch_bounds__(256)
-add_bias_rows_kernel(float* __restrict__ x, const float* __restrict__ bias, int H) {
+add_bias_rows_kernel(float* x, const float* __restrict__ bias, int H) {
   pdl_launch_dependents();
   pdl_wait();
   const size_t t = blockIdx.x;
@@ -376,7 +376,7 @@ softcap_rows_kernel(float* __restrict__ x, long long n, float cap) {
 // One block a row, a warp a head at a time.
 template <typename T>
 __global__ void __launch_bounds__(128)
-rotate_heads_kernel(T* __restrict__ x, int ldx, const int* __restrict__ positions, const float* __restrict__ inv_freq,
+rotate_heads_kernel(T* x, int ldx, const int* __restrict__ positions, const float* __restrict__ inv_freq,
                     int n, int interleaved, float sign, int nh, int HD) {
   extern __shared__ __align__(16) float cs[];        // n/2 cosines, n/2 sines
   pdl_launch_dependents();
@@ -405,7 +405,7 @@ rotate_heads_kernel(T* __restrict__ x, int ldx, const int* __restrict__ position
 
 // qkv rows [.. q: n_q floats at q_base ..]; z rows [heads*dk] become the decays.
 __global__ void __launch_bounds__(256)
-gla_prepare_kernel(float* __restrict__ qkv, int channels, int q_base, int n_q, float qscale, float* __restrict__ z,
+gla_prepare_kernel(float* qkv, int channels, int q_base, int n_q, float qscale, float* z,
                    const float* __restrict__ bias, int n_z, float inv_tau) {
   pdl_launch_dependents();
   pdl_wait();

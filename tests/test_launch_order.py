@@ -80,3 +80,24 @@ def test_only_constants_are_read_before_the_wait(name, params, body, structs):
             continue                                        # (an address is formed)
         for d in data:
             assert not re.search(d + r"\s*(\[|,|\+)|\*" + d.replace(r"(?<![\w.])", "") + r"\b", statement), f"before the wait: {statement.strip()}"
+
+
+# What `__restrict__` may promise of such a kernel: that nothing writes the data while the kernel is there.  It is there before
+# the kernel before it has ended, so that holds of the constants alone.
+PROMISED = CONSTANTS | {"ids", "prev", "table", "pair", "place", "bias", "conv_w", "a_log", "dt_bias", "skip_coef", "coef", "alpha", "sink",
+                        "temperature", "seed", "request_id", "position"}
+PROMISED_OF = {"dyt_norm_kernel": {"b"}, "dyt_norm_vec_kernel": {"b"}}
+STEP_TABLE = {"rope_cache_table_kernel"}                    # its table of angles is the step's
+
+
+@pytest.mark.parametrize("name,params,body,structs", EARLY)
+def test_restrict_qualifies_constants_and_results_only(name, params, body, structs):
+    for p in params:
+        arg = p.split()[-1]
+        if "__restrict__" not in p:
+            continue
+        if p.startswith("const "):
+            assert arg in (PROMISED - ({"table"} if name in STEP_TABLE else set())) | PROMISED_OF.get(name, set()), p
+        else:
+            assert not re.search(r"\b%s\[[^;=]*\]\s*[-+*/]=" % arg, body), f"{p}: changed in place"
+    assert not re.search(r"const\s+\w+\*\s*__restrict__\s+(qkv|state)\b", body)
