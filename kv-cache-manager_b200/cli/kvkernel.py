@@ -110,7 +110,7 @@ def bench_gemm(a, out) -> None:
             if K.stream_gemm_supported(M, N, Kd):
                 res["stream"] = graph_time_us([(lambda w=w: K.gemm_stream(x, w, y)) for w in ws])
             if K.splitk_gemm_supported(x, ws[0]):
-                res["splitk"] = graph_time_us([(lambda w=w: K.gemm_tcgen05_splitk(x, w, y)) for w in ws])
+                res["splitk"] = graph_time_us([(lambda w=w: K.gemm_tcgen05_splitk(x, w, y, weights_ready=True)) for w in ws])
             gb = N * Kd * 2 / 1e9
             print(f"M={M:<3} {name:<8} [{N} x {Kd}] " +
                   "  ".join(f"{k} {v:.1f} us ({gb / (v * 1e-6) / 1e3:.2f} TB/s)" for k, v in res.items()))

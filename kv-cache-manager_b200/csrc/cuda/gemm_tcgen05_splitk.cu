@@ -11,8 +11,8 @@
 // adds the S partial sums (always in block order: reproducible) of its share of the batch rows through
 // distributed shared memory, a warp a row, and ends the row (see SplitkEpilogue).
 //  * Two blocks share an SM (half of its shared memory and registers each).  Launched as programmatic dependents,
-//    they fill their rings with W (a constant) while what lies before still runs; X follows after the dependency
-//    wait.  (Blocks of 384 threads needed one SM each and were a quarter slower.)
+//    they fill their rings with W, where the caller vouches that it is a constant, while what lies before still runs; X
+//    follows after the dependency wait.  (Blocks of 384 threads needed one SM each and were a quarter slower.)
 //  * The residual stream and its norm ride along as in the weight-streaming kernel (gemm_stream.cu): a product
 //    that ends a sublayer adds into the float residual and leaves bfloat16(w * x_new) and, per tile of 128
 //    columns and row, the sum of squares; the product that begins the next one scales its sums by 1/rms.
@@ -59,6 +59,7 @@ enum SplitkEpilogue { kSkStore = 0, kSkRope = 1, kSkSilu = 2, kSkResidual = 3 };
 
 struct SplitkParams {
   void* Y; int M, N, K, ldy, Mp, stages, tmem_cols;
+  int weights_ready;                          // nothing that may still be running writes W
   // SCALED: the sums of row m are multiplied by rsqrt(sum over t of ss_in[t][m] / K + eps) before the epilogue
   const float* ss_in; int ss_tiles; float eps;
   // kSkRope: table [M][hd] (hd/2 cosines, then hd/2 sines)
@@ -133,8 +134,9 @@ gemm_tcgen05_splitk_kernel(const __grid_constant__ CUtensorMap map_w, const __gr
         tc5::tma_load_2d(smem_raw + size_t(s) * stage_bytes + kSkWBytes, &map_x, &full[s], (k_begin + i) * kSkBK, 0);
       };
       const int first = min(steps, stages);
-      for (int i = 0; i < first; ++i) load_w(i, i);            // weights are constants
-      pdl_wait();                                              // ... the predecessor wrote X
+      if (!p.weights_ready) pdl_wait();
+      for (int i = 0; i < first; ++i) load_w(i, i);
+      pdl_wait();                                              // (X is the predecessor's in any case)
       for (int i = 0; i < first; ++i) load_x(i, i);
       int issued = first;
       for (int i = first, s = 0, round = 1; i < steps && !abort_flag; ++i) {
@@ -385,18 +387,19 @@ KVCM_API int kvcm_gemm_tcgen05_splitk_supports(int M, int N, int K, int ldx, int
   return M >= 1 && M <= 256 && N >= 1 && K >= 8 && (K % 8) == 0 && (ldx % 8) == 0 && (ldw % 8) == 0;
 }
 
-// out_f32: 0 = bfloat16 result, 1 = float result.
+// out_f32: 0 = bfloat16 result, 1 = float result.  weights_ready = 1: nothing that is still running on the stream writes W
+// (a model's weights), so that it may be read before the launch's dependencies are done.
 KVCM_API int kvcm_gemm_tcgen05_splitk_bf16(const void* X, const void* W, void* Y, int M, int N, int K, int ldx, int ldw,
-                                           int ldy, int out_f32, void* stream) {
+                                           int ldy, int out_f32, int weights_ready, void* stream) {
   if (M == 0 || N == 0) return 0;
   if (!kvcm_gemm_tcgen05_splitk_supports(M, N, K, ldx, ldw) || !aligned16(X) || !aligned16(W)) return KVCM_ERR_UNSUPPORTED;
   SplitkParams p = {};
-  p.Y = Y; p.M = M; p.N = N; p.K = K; p.ldy = ldy;
+  p.Y = Y; p.M = M; p.N = N; p.K = K; p.ldy = ldy; p.weights_ready = weights_ready;
   cudaStream_t s = (cudaStream_t)stream;
   return out_f32 ? launch_splitk<float, kSkStore, false>(X, W, ldx, ldw, p, s) : launch_splitk<bf16, kSkStore, false>(X, W, ldx, ldw, p, s);
 }
 
-// The forms with a fused end, for a step of M rows of a model of these sizes (at most 128 rows: the partial sums of
+// The forms with a fused end (W is a model's weights: it is read ahead), for a step of M rows of a model of these sizes (at most 128 rows: the partial sums of
 // squares are kSkNormRows rows wide).
 KVCM_API int kvcm_splitk_fused_supports(int M, int N, int K) {
   return M >= 1 && M <= kSkNormRows && N >= 4 && (N % 4) == 0 && K >= 8 && (K % 8) == 0;
@@ -412,7 +415,7 @@ KVCM_API int kvcm_splitk_residual_bf16(const void* X, const void* W, float* resi
       !aligned16(resid) || !aligned16(h_out) || ss_out == nullptr || (next_w != nullptr && h_out == nullptr))
     return KVCM_ERR_UNSUPPORTED;
   SplitkParams p = {};
-  p.M = M; p.N = N; p.K = K;
+  p.M = M; p.N = N; p.K = K; p.weights_ready = 1;
   p.resid = resid; p.ldr = ldr; p.ss_out = ss_out; p.h_out = (bf16*)h_out; p.ldh = ldh; p.next_w = (const bf16*)next_w;
   return launch_splitk<bf16, kSkResidual, false>(X, W, ldx, ldw, p, (cudaStream_t)stream);
 }
@@ -428,7 +431,7 @@ KVCM_API int kvcm_splitk_qkv_bf16(const void* X, const float* ss_in, int ss_tile
       (ldy % 4) || !aligned16(X) || !aligned16(Wqkv) || !aligned16(Yq) || !aligned16(rope_table) || !aligned16(k_cache) || !aligned16(v_cache))
     return KVCM_ERR_UNSUPPORTED;
   SplitkParams p = {};
-  p.Y = Yq; p.M = M; p.N = N; p.K = K; p.ldy = ldy;
+  p.Y = Yq; p.M = M; p.N = N; p.K = K; p.ldy = ldy; p.weights_ready = 1;
   p.ss_in = ss_in; p.ss_tiles = ss_tiles; p.eps = eps;
   p.rope_table = rope_table; p.slot_mapping = slot_mapping; p.k_cache = (bf16*)k_cache; p.v_cache = (bf16*)v_cache;
   p.nh = nh; p.nkv = nkv; p.hd = hd; p.block_size = block_size;
@@ -443,7 +446,7 @@ KVCM_API int kvcm_splitk_gate_up_silu_bf16(const void* X, const float* ss_in, in
   if (!kvcm_splitk_fused_supports(M, I, K) || (ldx % 8) || (ldw % 8) || (ldy % 4) || !aligned16(X) || !aligned16(W) || !aligned16(Y))
     return KVCM_ERR_UNSUPPORTED;
   SplitkParams p = {};
-  p.Y = Y; p.M = M; p.N = I; p.K = K; p.ldy = ldy;
+  p.Y = Y; p.M = M; p.N = I; p.K = K; p.ldy = ldy; p.weights_ready = 1;
   p.ss_in = ss_in; p.ss_tiles = ss_tiles; p.eps = eps;
   cudaStream_t s = (cudaStream_t)stream;
   return ss_in ? launch_splitk<bf16, kSkSilu, true>(X, W, ldx, ldw, p, s) : launch_splitk<bf16, kSkSilu, false>(X, W, ldx, ldw, p, s);

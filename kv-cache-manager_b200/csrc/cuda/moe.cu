@@ -354,13 +354,14 @@ moe_route_mma_kernel(const bf16* h, int ldh, const bf16* __restrict__ wr, int ro
 
 // The same for a step of few rows, which one block would walk through in one latency after another: the width is split
 // over the eight blocks of a cluster, so that at a width of 2,048 every warp has one block of 32 columns, whose router rows it
-// asks for before the dependency wait (they are weights).  The blocks' sums (over their warps in order) meet in distributed
+// asks for before the dependency wait (where the caller
+// vouches that they are weights).  The blocks' sums (over their warps in order) meet in distributed
 // shared memory; block r adds them in the order of the blocks and chooses for rows r and r + 8.  At most 8 * NT outputs.
 // Four rows of 2,048 columns, 33 outputs, in a decode step: 6.9 us, one block of eight warps 12.8.
 constexpr int ROUTE_SPLIT = 8;
 template <int NT>
 __global__ void __launch_bounds__(ROUTE_WARPS * 32)
-moe_route_few_kernel(const bf16* h, int ldh, const bf16* __restrict__ wr, int rows, int D, RouteChoice choice) {
+moe_route_few_kernel(const bf16* h, int ldh, const bf16* __restrict__ wr, int rows, int D, int weights_ready, RouteChoice choice) {
   constexpr int NP = 8 * NT;
   extern __shared__ __align__(16) float route_smem[];       // [2] rows of a choice | [warps][16][NP] | [16][NP]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t4 = lane & 3;
@@ -380,7 +381,8 @@ moe_route_few_kernel(const bf16* h, int ldh, const bf16* __restrict__ wr, int ro
   const bf16* ra = h + size_t(min(row0 + g, rows - 1)) * ldh + t4 * 8;
   const bf16* rb = h + size_t(min(row0 + g + 8, rows - 1)) * ldh + t4 * 8;
   pdl_launch_dependents();
-  bool waited = false;
+  bool waited = !weights_ready;
+  if (waited) pdl_wait();
   for (int kb = (rank * ROUTE_WARPS + warp) * 32; kb < D; kb += ROUTE_SPLIT * ROUTE_WARPS * 32) {
     const bool in = kb + t4 * 8 < D;                        // (D % 8 == 0)
     uint4 w[NT];
@@ -686,7 +688,7 @@ moe_combine_kernel(const float* y, const int* place_of, const float* wt, int top
 template <typename T>
 int launch_moe_route(const void* h, int ldh, const void* wr, int w_f32, int rows, int D, int E, int G, int keep, int top,
                      float scale, int has_gate, int scores, const float* bias, const float* correction, int group_top, int renorm, int* idx,
-                     float* wt, float* gate_out, cudaStream_t s) {
+                     float* wt, float* gate_out, int weights_ready, cudaStream_t s) {
   if (rows == 0) return 0;
   if (E < 1 || G < 1 || E % G || keep < 1 || keep > G || top < 1 || top > (E / G) * keep || group_top < 1 || group_top > 2 || scores < 0 || scores > 2)
     return KVCM_ERR_UNSUPPORTED;
@@ -707,7 +709,7 @@ int launch_moe_route(const void* h, int ldh, const void* wr, int w_f32, int rows
       if (rows <= 4 * ROUTE_MMA_ROWS && outs <= np && few_smem <= 48 * 1024) {
         auto few = np == 32 ? moe_route_few_kernel<4> : np == 40 ? moe_route_few_kernel<5> : moe_route_few_kernel<8>;
         return pdl_launch_cluster(few, dim3(grid.x * ROUTE_SPLIT), dim3(ROUTE_WARPS * 32), few_smem, s, ROUTE_SPLIT, (const bf16*)h, ldh,
-                                  (const bf16*)wr, rows, D, choice);
+                                  (const bf16*)wr, rows, D, weights_ready, choice);
       }
       auto kernel = np == 32 ? moe_route_mma_kernel<4> : np == 40 ? moe_route_mma_kernel<5> : moe_route_mma_kernel<8>;
       if (mma_smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mma_smem);
@@ -819,9 +821,9 @@ KVCM_API int kvcm_moe_experts_tc_bf16(const void* h, int ldh, const void* wgu, c
   KVCM_API int kvcm_moe_route_##SUFFIX(const void* h, int ldh, const void* wr, int w_f32, int rows, int D, int E,    \
                                        int G, int keep, int top, float scale, int has_gate, int scores,              \
                                        const float* bias, const float* correction, int group_top, int renorm, int* idx, float* wt, \
-                                       float* gate_out, void* stream) {                                              \
+                                       float* gate_out, int weights_ready, void* stream) {                           \
     return launch_moe_route<T>(h, ldh, wr, w_f32, rows, D, E, G, keep, top, scale, has_gate, scores, bias,           \
-                               correction, group_top, renorm, idx, wt, gate_out, (cudaStream_t)stream);              \
+                               correction, group_top, renorm, idx, wt, gate_out, weights_ready, (cudaStream_t)stream); \
   }                                                                                                                  \
   KVCM_API int kvcm_moe_experts_##SUFFIX(const void* h, int ldh, const void* wgu, const void* wd, const int* idx,    \
                                          int rows, int top, int E, int F, int D, int* work, void* act, float* y,     \

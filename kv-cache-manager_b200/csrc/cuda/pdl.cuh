@@ -7,9 +7,10 @@
 // ordinary way simply waits for full completion, so mixing both kinds is always correct.
 // Rules for a kernel launched through pdl_launch:
 //  * It writes global memory only after pdl_wait().
-//  * Before pdl_wait() it reads constants only: weights (of a caller that vouches for them, `weights_ready`), what a
-//    completed copy or an earlier step wrote (the batch's integers, keys and values of earlier tokens).  Data of the same
-//    step, however many launches back it was written, is read after the wait: nothing else makes it visible here.
+//  * Before pdl_wait() it reads constants only: weights (of a caller that vouches for them, `weights_ready`; the streaming
+//    products and the products with fused ends take nothing else as W), and what a completed copy or an earlier step wrote
+//    (the batch's integers, keys and values of earlier tokens).  Data of the same step, however many launches back it was
+//    written, is read after the wait: nothing else makes it visible here.
 //  * `__restrict__` qualifies constants and results only.  It promises that nobody writes the data while the kernel is
 //    there, which allows loads to be moved across the wait and through caches that are not coherent; but the kernel is
 //    there while the one before still writes.

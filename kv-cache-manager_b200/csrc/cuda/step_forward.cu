@@ -68,7 +68,7 @@ int kvcm_qkv_rope_cache_scaled_bf16(const void*, const float*, int, float, const
 int kvcm_gate_up_silu_scaled_bf16(const void*, const float*, int, float, const void*, void*, int, int, int, int, int, int, int,
                                   void*);
 int kvcm_gemm_tcgen05_splitk_supports(int, int, int, int, int);
-int kvcm_gemm_tcgen05_splitk_bf16(const void*, const void*, void*, int, int, int, int, int, int, int, void*);
+int kvcm_gemm_tcgen05_splitk_bf16(const void*, const void*, void*, int, int, int, int, int, int, int, int, void*);
 int kvcm_splitk_fused_supports(int, int, int);
 long long kvcm_splitk_norm_floats(int);
 int kvcm_splitk_residual_bf16(const void*, const void*, float*, float*, void*, const void*, int, int, int, int, int, int, int, void*);
@@ -139,7 +139,7 @@ int product(const KvcmForwardArgs& a, const void* x, const void* w, void* y, int
     return kvcm_gemm_stream_bf16(x, w, y, M, N, K, K, K, N, out_f32 ? 1 : 0, a.sm_count, s);
   if (M <= kSplitkMaxRows && kvcm_gemm_tcgen05_splitk_supports(M, N, K, K, K) &&
       ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) == 0)
-    return kvcm_gemm_tcgen05_splitk_bf16(x, w, y, M, N, K, K, K, N, out_f32 ? 1 : 0, s);
+    return kvcm_gemm_tcgen05_splitk_bf16(x, w, y, M, N, K, K, K, N, out_f32 ? 1 : 0, 1, s);
   return library_gemm(a, x, w, y, M, N, K, out_f32, s);
 }
 

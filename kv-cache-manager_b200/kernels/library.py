@@ -786,11 +786,12 @@ def splitk_gemm_supported(x: torch.Tensor, w: torch.Tensor) -> bool:
             and bool(_lib().kvcm_gemm_tcgen05_splitk_supports(x.shape[0], w.shape[0], x.shape[1], x.stride(0), w.stride(0))))
 
 
-def gemm_tcgen05_splitk(x: torch.Tensor, w: torch.Tensor, y: torch.Tensor) -> None:
+def gemm_tcgen05_splitk(x: torch.Tensor, w: torch.Tensor, y: torch.Tensor, weights_ready: bool = False) -> None:
     """y[M,N] = x[M,K] @ w[N,K]^T for M <= 256 on the fifth-generation tensor cores with the operands
     swapped (128 weight rows are the tall operand) and K split over a thread-block cluster whose
     blocks add their partial sums through distributed shared memory.  bfloat16 operands; bfloat16 or
-    float32 result."""
+    float32 result.  ``weights_ready``: nothing that is still running on the stream writes ``w`` (a model's weights), so that
+    it may be read before the launches in front of this one are done."""
     _cuda(x, w, y)
     M, K = x.shape
     N = w.shape[0]
@@ -799,7 +800,7 @@ def gemm_tcgen05_splitk(x: torch.Tensor, w: torch.Tensor, y: torch.Tensor) -> No
           "gemm_tcgen05_splitk: bfloat16 operands, bfloat16 or float32 result")
     _need(x.stride(1) == 1 and w.stride(1) == 1 and y.stride(1) == 1, "gemm_tcgen05_splitk: rows must be dense")
     rc = _lib().kvcm_gemm_tcgen05_splitk_bf16(_p(x), _p(w), _p(y), M, N, K, x.stride(0), w.stride(0), y.stride(0),
-                                              int(y.dtype == torch.float32), _stream())
+                                              int(y.dtype == torch.float32), int(weights_ready), _stream())
     _check(rc, "gemm_tcgen05_splitk", f"(M={M}, N={N}, K={K})")
 
 
@@ -1108,13 +1109,14 @@ ROUTE_SCORES = {"softmax": 0, "sigmoid": 1, "softmax_chosen": 2}
 def moe_route(h: torch.Tensor, router: torch.Tensor, experts: int, groups: int, keep: int, top: int, scale: float,
               idx: torch.Tensor, wt: torch.Tensor, gate: Optional[torch.Tensor], scores: str = "softmax",
               correction: Optional[torch.Tensor] = None, group_top: int = 1, renorm: bool = False,
-              bias: Optional[torch.Tensor] = None) -> None:
+              bias: Optional[torch.Tensor] = None, weights_ready: bool = False) -> None:
     """Per row: float32 router logits (plus ``bias``, float32 [experts]), scores (``scores``: "softmax" over all experts, "sigmoid" of
     each logit, or "softmax_chosen": the largest logits are chosen and their softmax among themselves are the weights), group-limited choice of ``top`` experts; ``idx`` int32 [T, top], ``wt`` float32 [T, top] =
     score * scale; ``gate`` float32 [T] = sigmoid of the logit of the router matrix's extra row (row
     ``experts``).  ``correction`` (float32 [experts]) is added to the scores for the choice only;
     ``group_top``: a group's score is the sum of its 1 or 2 largest choice scores; ``renorm``: the chosen scores are
-    divided by their sum (+ 1e-20) before the scale."""
+    divided by their sum (+ 1e-20) before the scale.  ``weights_ready``: nothing that is still running on the stream writes
+    ``router`` (a model's weights), so that it may be read before the launches in front of this one are done."""
     _cuda(h, router, idx, wt, gate, correction)
     _need(scores in ROUTE_SCORES and group_top in (1, 2), "moe_route: scores 'softmax' | 'sigmoid' | 'softmax_chosen', group_top 1 | 2")
     _need(bias is None or (bias.dtype == torch.float32 and bias.is_contiguous() and bias.numel() == experts and bias.is_cuda),
@@ -1130,7 +1132,7 @@ def moe_route(h: torch.Tensor, router: torch.Tensor, experts: int, groups: int, 
     fn = getattr(_lib(), "kvcm_moe_route_" + _suffix(h))
     _check(fn(_p(h), h.stride(0), _p(router), int(router.dtype == torch.float32), T, D, experts, groups, keep, top,
               ctypes.c_float(scale), int(gate is not None), ROUTE_SCORES[scores], _p(bias), _p(correction), int(group_top),
-              int(bool(renorm)), _p(idx), _p(wt), _p(gate), _stream()), "moe_route",
+              int(bool(renorm)), _p(idx), _p(wt), _p(gate), int(weights_ready), _stream()), "moe_route",
            f"(experts={experts}, groups={groups}, keep={keep}, top={top})")
 
 

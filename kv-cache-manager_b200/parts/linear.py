@@ -84,7 +84,7 @@ def matmul_nt(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype, options:
     # tcgen05 kernel: correct and reproducible, about half the library's speed at these sizes).
     if (native or mode == "splitk") and K.splitk_gemm_supported(x, w):
         y = torch.empty((M, N), dtype=out_dtype, device=x.device)
-        K.gemm_tcgen05_splitk(x, w, y)
+        K.gemm_tcgen05_splitk(x, w, y, weights_ready=True)
         return y
     y = torch.mm(x, w.t()) if out_dtype == torch.bfloat16 else torch.mm(x, w.t(), out_dtype=out_dtype)
     K.profile_mark("library_gemm")

@@ -97,7 +97,7 @@ class RoutedExperts(FeedForward):
         wt = torch.empty((M, top), dtype=torch.float32, device=dev)
         gate = torch.empty((M,), dtype=torch.float32, device=dev) if self.shared_gate else None
         K.moe_route(h, self._router, self.experts, self.groups, self.keep, top, self.scale, idx, wt, gate, self.scores,
-                    self._correction, self.group_top, self.renorm, self._bias)
+                    self._correction, self.group_top, self.renorm, self._bias, weights_ready=True)
         work = torch.empty((K.moe_work_ints(M, top, self.experts),), dtype=torch.int32, device=dev)
         act = torch.empty((M * top, self.expert_ff), dtype=h.dtype, device=dev)
         y = torch.empty((M * top, D), dtype=torch.float32, device=dev)

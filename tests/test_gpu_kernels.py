@@ -171,6 +171,32 @@ def test_float32_product_at_the_edges_of_its_tiles(M, N, Kd, ld):
     assert torch.equal(one, y[M - 1:])
 
 
+def test_operands_written_by_the_launch_in_front_are_waited_for():
+    """Weights that the kernel in front writes (it lets its dependents start before it has written anything): the split-K
+    product and the router wait for them unless the caller vouches for them.  Against the same launches one at a time."""
+    lib = K()
+    g = torch.Generator(device=DEV).manual_seed(4)
+    M, N, Kd, E, top = 24, 4096, 2048, 40, 4
+    x = torch.randn(M, Kd, generator=g, device=DEV).to(torch.bfloat16)
+    srcs = [torch.randn(N, Kd, generator=g, device=DEV) for _ in range(12)]
+    w = torch.empty(N, Kd, dtype=torch.bfloat16, device=DEV)
+
+    def run(one_at_a_time):
+        out = []
+        for s in srcs:
+            y, wt = torch.empty(M, N, device=DEV), torch.empty(M, top, device=DEV)
+            idx = torch.empty(M, top, dtype=torch.int32, device=DEV)
+            for step in (lambda: lib.cast_rows(s, w), lambda: lib.gemm_tcgen05_splitk(x, w, y),
+                         lambda: lib.cast_rows(s[N - E:], w[:E]), lambda: lib.moe_route(x, w[:E], E, 1, 1, top, 1.0, idx, wt, None)):
+                step()
+                if one_at_a_time:
+                    torch.cuda.synchronize()
+            out += [y, idx, wt]
+        return out
+    for a, b in zip(run(False), run(True)):
+        assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("M,N,Kd", [(1, 2048, 2048), (8, 2560, 2048), (3, 100, 176), (16, 37, 2048), (8, 37, 5632),
                                     (9, 515, 96), (8, 32003, 256), (5, 16, 8), (8, 11264, 2048),
                                     (7, 4096, 1032), (2, 33, 520),
