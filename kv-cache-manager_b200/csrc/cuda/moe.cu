@@ -20,8 +20,11 @@
 //
 // Nothing is read on the host: counts and tile lists stay on the device and the product grids
 // are sized for the worst case (pairs / 64 + experts tiles), so a step can be recorded into a
-// CUDA graph.  Every output element is accumulated by one thread over k in ascending order, so
-// a row's result does not depend on what else is in the batch or on the order inside a tile.
+// CUDA graph.  Here every output element is accumulated by one thread over k in ascending order, so
+// a row's result does not depend on what else is in the batch or on the order inside a tile; the
+// bfloat16 router too takes one order of summation whatever the number of rows, so a row's choice
+// does not depend on it.  (The experts' products of bfloat16 rows differ in their order of
+// summation between the forms, that is, between steps of up to 16 rows and longer ones.)
 // Instantiated for float (the true 32-bit path: float FMAs only) and bfloat16 storage.
 #include <cooperative_groups.h>
 
@@ -352,76 +355,70 @@ moe_route_mma_kernel(const bf16* h, int ldh, const bf16* __restrict__ wr, int ro
   }
 }
 
-// The same for a step of few rows, which one block would walk through in one latency after another: the width is split
-// over the eight blocks of a cluster, so that at a width of 2,048 every warp has one block of 32 columns, whose router rows it
-// asks for before the dependency wait (where the caller
-// vouches that they are weights).  The blocks' sums (over their warps in order) meet in distributed
-// shared memory; block r adds them in the order of the blocks and chooses for rows r and r + 8.  At most 8 * NT outputs.
-// Four rows of 2,048 columns, 33 outputs, in a decode step: 6.9 us, one block of eight warps 12.8.
-constexpr int ROUTE_SPLIT = 8;
+// The same for a step of few rows, which one block would walk through in one latency after another.  The same sums in the same
+// order, so that a row's choice does not depend on how many rows are beside it: what a warp sums up above is a block of a
+// cluster here, with a warp for every eight outputs.  At a width of 2,048 a warp has its eight blocks of 32 columns of the
+// router under way at once, asked for before the dependency wait where the caller vouches that they are weights.  The
+// blocks' sums meet in distributed shared memory; block r adds them in their order and chooses for rows r and r + 8.  At
+// most 8 * NT outputs.
+// Four rows of 2,048 columns, 33 outputs, in a decode step: @@ us, one block of eight warps 12.8.
+constexpr int ROUTE_AHEAD = 8;                              // blocks of 32 columns a warp has under way
 template <int NT>
-__global__ void __launch_bounds__(ROUTE_WARPS * 32)
+__global__ void __launch_bounds__(NT * 32)
 moe_route_few_kernel(const bf16* h, int ldh, const bf16* __restrict__ wr, int rows, int D, int weights_ready, RouteChoice choice) {
   constexpr int NP = 8 * NT;
-  extern __shared__ __align__(16) float route_smem[];       // [2] rows of a choice | [warps][16][NP] | [16][NP]
+  extern __shared__ __align__(16) float route_smem[];       // [2] rows of a choice | [16][NP] this block's sums
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t4 = lane & 3;
-  const int row0 = int(blockIdx.x) / ROUTE_SPLIT * ROUTE_MMA_ROWS, rank = int(blockIdx.x) % ROUTE_SPLIT;
+  const int row0 = int(blockIdx.x) / ROUTE_WARPS * ROUTE_MMA_ROWS, rank = int(blockIdx.x) % ROUTE_WARPS;
   const int E = choice.E, outs = E + (choice.has_gate ? 1 : 0);
   const int zstride = (2 * E + 1 + choice.G + 3) & ~3;
-  float* part = route_smem + 2 * zstride;
-  float* sums = part + ROUTE_WARPS * ROUTE_MMA_ROWS * NP;
+  float* sums = route_smem + 2 * zstride;
   const uint4 none = make_uint4(0u, 0u, 0u, 0u);
-  float acc[NT][4];
-  const bf16* we[NT];
-#pragma unroll
-  for (int i = 0; i < NT; ++i) {
-    acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
-    we[i] = wr + size_t(min(8 * i + g, outs - 1)) * D + t4 * 8;
-  }
+  const bf16* we = wr + size_t(min(8 * warp + g, outs - 1)) * D + t4 * 8;
   const bf16* ra = h + size_t(min(row0 + g, rows - 1)) * ldh + t4 * 8;
   const bf16* rb = h + size_t(min(row0 + g + 8, rows - 1)) * ldh + t4 * 8;
   pdl_launch_dependents();
   bool waited = !weights_ready;
   if (waited) pdl_wait();
-  for (int kb = (rank * ROUTE_WARPS + warp) * 32; kb < D; kb += ROUTE_SPLIT * ROUTE_WARPS * 32) {
-    const bool in = kb + t4 * 8 < D;                        // (D % 8 == 0)
-    uint4 w[NT];
+  float acc[4] = {0.f, 0.f, 0.f, 0.f};
+  for (int k0 = rank * 32; k0 < D; k0 += ROUTE_AHEAD * ROUTE_WARPS * 32) {
+    uint4 w[ROUTE_AHEAD], a[ROUTE_AHEAD], b[ROUTE_AHEAD];
 #pragma unroll
-    for (int i = 0; i < NT; ++i) w[i] = in ? *reinterpret_cast<const uint4*>(we[i] + kb) : none;
+    for (int u = 0; u < ROUTE_AHEAD; ++u) {
+      const int k = k0 + u * ROUTE_WARPS * 32;
+      w[u] = k + t4 * 8 < D ? *reinterpret_cast<const uint4*>(we + k) : none;          // (D % 8 == 0)
+    }
     if (!waited) { pdl_wait(); waited = true; }
-    const uint4 a = in ? *reinterpret_cast<const uint4*>(ra + kb) : none, b = in ? *reinterpret_cast<const uint4*>(rb + kb) : none;
 #pragma unroll
-    for (int i = 0; i < NT; ++i) {
-      route_mma(acc[i], a.x, b.x, a.y, b.y, w[i].x, w[i].y);
-      route_mma(acc[i], a.z, b.z, a.w, b.w, w[i].z, w[i].w);
+    for (int u = 0; u < ROUTE_AHEAD; ++u) {
+      const int k = k0 + u * ROUTE_WARPS * 32;
+      const bool in = k + t4 * 8 < D;
+      a[u] = in ? *reinterpret_cast<const uint4*>(ra + k) : none;
+      b[u] = in ? *reinterpret_cast<const uint4*>(rb + k) : none;
+    }
+#pragma unroll
+    for (int u = 0; u < ROUTE_AHEAD; ++u) {
+      if (k0 + u * ROUTE_WARPS * 32 >= D) break;
+      route_mma(acc, a[u].x, b[u].x, a[u].y, b[u].y, w[u].x, w[u].y);
+      route_mma(acc, a[u].z, b[u].z, a[u].w, b[u].w, w[u].z, w[u].w);
     }
   }
   if (!waited) pdl_wait();                                  // before anything is written
-#pragma unroll
-  for (int i = 0; i < NT; ++i) {
-    float* at = part + (warp * ROUTE_MMA_ROWS + g) * NP + 8 * i + 2 * t4;
-    at[0] = acc[i][0]; at[1] = acc[i][1];
-    at[8 * NP] = acc[i][2]; at[8 * NP + 1] = acc[i][3];
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < ROUTE_MMA_ROWS * NP; i += ROUTE_WARPS * 32) {
-    float z = 0.f;
-#pragma unroll
-    for (int w = 0; w < ROUTE_WARPS; ++w) z += part[w * ROUTE_MMA_ROWS * NP + i];
-    sums[i] = z;
-  }
+  float* at = sums + g * NP + 8 * warp + 2 * t4;
+  at[0] = acc[0]; at[1] = acc[1];
+  at[8 * NP] = acc[2]; at[8 * NP + 1] = acc[3];
   const auto cluster = cooperative_groups::this_cluster();
   cluster.sync();
-  const int local = rank + ROUTE_SPLIT * warp, row = row0 + local;
-  if (warp < ROUTE_MMA_ROWS / ROUTE_SPLIT && row < rows) {
+  const int local = rank + ROUTE_WARPS * warp, row = row0 + local;
+  if (warp < ROUTE_MMA_ROWS / ROUTE_WARPS && row < rows) {
     float* z = route_smem + warp * zstride;
     for (int e = lane; e < outs; e += 32) {
-      float v[ROUTE_SPLIT];
+      float v[ROUTE_WARPS];
 #pragma unroll
-      for (int r = 0; r < ROUTE_SPLIT; ++r) v[r] = *cluster.map_shared_rank(sums + local * NP + e, r);
-      float t = v[0];
+      for (int r = 0; r < ROUTE_WARPS; ++r) v[r] = *cluster.map_shared_rank(sums + local * NP + e, r);
+      float t = 0.f;
 #pragma unroll
-      for (int r = 1; r < ROUTE_SPLIT; ++r) t += v[r];
+      for (int r = 0; r < ROUTE_WARPS; ++r) t += v[r];
       z[e] = t;
     }
     __syncwarp();
@@ -704,11 +701,11 @@ int launch_moe_route(const void* h, int ldh, const void* wr, int w_f32, int rows
     if (!w_f32 && (D % 8) == 0 && (ldh % 8) == 0 && ((reinterpret_cast<uintptr_t>(h) | reinterpret_cast<uintptr_t>(wr)) & 15) == 0 &&
         mma_smem <= 200 * 1024) {
       const dim3 grid((rows + ROUTE_MMA_ROWS - 1) / ROUTE_MMA_ROWS);
-      const size_t few_smem = (2 * zstride + (ROUTE_WARPS + 1) * ROUTE_MMA_ROWS * np) * sizeof(float);
+      const size_t few_smem = (2 * zstride + ROUTE_MMA_ROWS * np) * sizeof(float);
       // up to four clusters; with more rows the blocks of sixteen fill SMs by themselves
       if (rows <= 4 * ROUTE_MMA_ROWS && outs <= np && few_smem <= 48 * 1024) {
         auto few = np == 32 ? moe_route_few_kernel<4> : np == 40 ? moe_route_few_kernel<5> : moe_route_few_kernel<8>;
-        return pdl_launch_cluster(few, dim3(grid.x * ROUTE_SPLIT), dim3(ROUTE_WARPS * 32), few_smem, s, ROUTE_SPLIT, (const bf16*)h, ldh,
+        return pdl_launch_cluster(few, dim3(grid.x * ROUTE_WARPS), dim3(np * 4), few_smem, s, ROUTE_WARPS, (const bf16*)h, ldh,
                                   (const bf16*)wr, rows, D, weights_ready, choice);
       }
       auto kernel = np == 32 ? moe_route_mma_kernel<4> : np == 40 ? moe_route_mma_kernel<5> : moe_route_mma_kernel<8>;

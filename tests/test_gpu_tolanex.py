@@ -564,6 +564,46 @@ def test_router_split_over_a_cluster_against_float64(T, E, D, gate):
         assert torch.allclose(out.double(), torch.sigmoid(z[:, E]), rtol=1e-4)
 
 
+@pytest.mark.parametrize("E,D,gate,top", [(8, 8, False, 3), (32, 2048, True, 8), (31, 72, False, 4), (39, 2056, True, 4), (60, 520, False, 6),
+                                          (33, 4136, False, 4)])
+def test_a_routed_row_does_not_depend_on_the_rows_beside_it(E, D, gate, top):
+    """The router takes one order of summation on both sides of its change of form (64 rows): the same bits.  The experts'
+    products do not at theirs (16 rows): float sums of D products and a bfloat16 activation, the bound of the products' own tests."""
+    from kvcm.kernels import library as K
+    g = torch.Generator().manual_seed(E + D)
+    T, F = 80, 40
+    h = torch.randn(T, D, generator=g).to(torch.bfloat16).cuda()
+    wr = (torch.randn(E + gate, D, generator=g) * 3 * D ** -0.5).to(torch.bfloat16).cuda()
+    wgu = (torch.randn(E, 2 * F, D, generator=g) * D ** -0.5).to(torch.bfloat16).cuda()
+    wd = (torch.randn(E, D, F, generator=g) * F ** -0.5).to(torch.bfloat16).cuda()
+
+    def route(rows):
+        n = rows.shape[0]
+        idx, wt = torch.empty(n, top, dtype=torch.int32, device="cuda"), torch.empty(n, top, device="cuda")
+        out = torch.empty(n, device="cuda") if gate else None
+        K.moe_route(rows, wr, E, 1, 1, top, 1.5, idx, wt, out)
+        return idx, wt, out
+
+    def experts(rows, idx, wt):
+        n = rows.shape[0]
+        work = torch.empty(K.moe_work_ints(n, top, E), dtype=torch.int32, device="cuda")
+        act, y = torch.empty(n * top, F, dtype=torch.bfloat16, device="cuda"), torch.empty(n * top, D, device="cuda")
+        out = torch.empty(n, D, device="cuda")
+        if K.moe_few_supported(rows, top, E, F):
+            K.moe_experts_few(rows, wgu, wd, idx, work, act, y)
+        else:
+            K.moe_experts(rows, wgu, wd, idx, work, act, y, torch.empty(n * top, D, dtype=torch.bfloat16, device="cuda"))
+        K.moe_combine(y, work, wt, E, None, None, out)
+        return out, y.std(correction=0).item()
+    whole = route(h)
+    for n in (1, 4, 16, 17, 63, 64, 65):
+        part = route(h[:n])
+        assert all(a is b is None or torch.equal(a, b[:n]) for a, b in zip(part, whole))
+    (a, std), (b, _) = (experts(h[:n], whole[0][:n], whole[1][:n]) for n in (16, 17))
+    # each form is within 0.04 standard deviations of the exact products; a row's weights add up to at most 1.5
+    assert (a - b[:16]).abs().max().item() <= 1.5 * 2 * 0.04 * std
+
+
 def test_score_borrows_a_state_slot(folders, oracle):
     """``Engine.score`` on a model with per-request state: teacher-forced logits of a whole sequence,
     twice (the slot is zeroed each time) and with requests running beside it."""
