@@ -9,6 +9,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "../include/once_per_device.h"
+
 #define KVCM_API extern "C" __attribute__((visibility("default")))
 #define KVCM_LAUNCH_RESULT() static_cast<int>(cudaGetLastError())
 
@@ -19,6 +21,15 @@
 namespace kvcm {
 
 typedef __nv_bfloat16 bf16;
+
+// Raises the limit of dynamic shared memory of a kernel on the current device.  `once` belongs to the kernel.
+template <typename Kernel>
+int allow_shared_memory(OncePerDevice& once, Kernel kernel, size_t bytes) {
+  int device = 0;
+  const cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return int(e);
+  return once(device, [&] { return int(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes))); });
+}
 
 template <typename T> struct Store;
 template <> struct Store<float> {

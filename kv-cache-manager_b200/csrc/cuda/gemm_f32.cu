@@ -178,8 +178,9 @@ static int segments(int K) { return K >= 1024 ? 8 : K >= 512 ? 4 : K >= 256 ? 2 
 template <typename C, bool VEC>
 static int launch_tile(const float* X, const float* W, float* Y, int M, int N, int K, int ldx, int ldw, int ldy, int weights_ready,
                        cudaStream_t s) {
-  static const cudaError_t attr = cudaFuncSetAttribute(gemm_f32_kernel<C, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
-  if (attr != cudaSuccess) return int(attr);
+  static OncePerDevice once;
+  const int rc = allow_shared_memory(once, gemm_f32_kernel<C, VEC>, C::SMEM);
+  if (rc) return rc;
   const int S = segments(K), seg = ((K + S - 1) / S + 3) / 4 * 4;
   const long long mtiles = (M + C::BM - 1) / C::BM, blocks = mtiles * ((N + C::BN - 1) / C::BN) * S;
   if (blocks > 0x7fffffffll) return KVCM_ERR_UNSUPPORTED;

@@ -369,11 +369,9 @@ int launch_splitk(const void* X, const void* W, int ldx, int ldw, SplitkParams p
   p.tmem_cols = 32;
   while (p.tmem_cols < p.Mp) p.tmem_cols *= 2;
   auto kernel = S <= 4 ? gemm_tcgen05_splitk_kernel<OutT, EPI, SCALED, 4> : gemm_tcgen05_splitk_kernel<OutT, EPI, SCALED, kSkMaxSplit>;
-  static const cudaError_t configured4 = cudaFuncSetAttribute(gemm_tcgen05_splitk_kernel<OutT, EPI, SCALED, 4>,
-                                                              cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSkSmemLimit));
-  static const cudaError_t configured8 = cudaFuncSetAttribute(gemm_tcgen05_splitk_kernel<OutT, EPI, SCALED, kSkMaxSplit>,
-                                                              cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSkSmemLimit));
-  if (configured4 != cudaSuccess || configured8 != cudaSuccess) return int(configured4 != cudaSuccess ? configured4 : configured8);
+  static OncePerDevice once[2];
+  rc = allow_shared_memory(once[S <= 4 ? 0 : 1], kernel, kSkSmemLimit);
+  if (rc) return rc;
   return pdl_launch_cluster(kernel, dim3(tiles * S), dim3(kSkThreads), smem, s, S, mw, mx, p);
 }
 
