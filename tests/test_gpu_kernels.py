@@ -836,6 +836,27 @@ def test_decode_attention_long_contexts_and_many_partitions():
         close(out, ref, "bfloat16", version)
 
 
+@pytest.mark.parametrize("hd,seqs", [(64, 40), (128, 24)])
+@pytest.mark.parametrize("lens", ["ragged", "equal"])
+def test_decode_attention_of_more_blocks_than_run_at_once(hd, seqs, lens):
+    """32 KV heads of `seqs` requests do not all run at once: the requests are then taken longest first, every block finding
+    its own.  Ragged lengths with ties and entries without a key, and equal lengths; undivided and in both merge forms."""
+    nh, g = 32, torch.Generator().manual_seed(seqs)
+    assert nh * seqs > K()._decode_resident_blocks(hd, DEV)
+    seq_lens = [130] * seqs
+    if lens == "ragged":
+        seq_lens = torch.randint(1, 330, (seqs,), generator=g).tolist()
+        seq_lens[3] = seq_lens[17] = 0
+        seq_lens[5] = seq_lens[6] = seq_lens[20] = 257
+    case = paged_case(seq_lens, [1] * seqs, nh, nh, hd, 16, "bfloat16", seed=hd)
+    ref = reference_attention(case, nh, nh, hd, hd ** -0.5, 0)
+    for options in ({"attn_version": "v1"}, {"attn_parts": 3}, {"attn_parts": 3, "attn_merge": "kernel"}):
+        case["ctx"].options = options
+        out = torch.full((seqs, nh * hd), float("nan"), dtype=torch.bfloat16, device=DEV)
+        K().attention_decode(case["q"], out, case["kc"], case["vc"], case["tables"], case["ctx"], nh, nh, hd, hd ** -0.5)
+        close(out, ref, "bfloat16", str(options))
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("needle", [0, 15, 16, 63, 64, 255, 256, 700, 998])
 def test_one_far_key_among_hundreds_decides_the_output(dtype, needle):
