@@ -361,7 +361,7 @@ moe_route_mma_kernel(const bf16* h, int ldh, const bf16* __restrict__ wr, int ro
 // router under way at once, asked for before the dependency wait where the caller vouches that they are weights.  The
 // blocks' sums meet in distributed shared memory; block r adds them in their order and chooses for rows r and r + 8.  At
 // most 8 * NT outputs.
-// Four rows of 2,048 columns, 33 outputs, in a decode step: @@ us, one block of eight warps 12.8.
+// Four rows of 2,048 columns, 33 outputs, launches back to back: 6.3 us, one block of eight warps 9.5 (in a decode step 12.8).
 constexpr int ROUTE_AHEAD = 8;                              // blocks of 32 columns a warp has under way
 template <int NT>
 __global__ void __launch_bounds__(NT * 32)
@@ -696,8 +696,8 @@ int launch_moe_route(const void* h, int ldh, const void* wr, int w_f32, int rows
   if (smem > 200 * 1024) return KVCM_ERR_UNSUPPORTED;
   const RouteChoice choice = {E, G, keep, top, has_gate, scores, group_top, renorm, scale, correction, bias, idx, wt, gate_out};
   if constexpr (sizeof(T) == 2) {
-    const int outs = E + (has_gate ? 1 : 0), np = outs <= 32 ? 32 : outs <= 40 ? 40 : 64;
-    const size_t mma_smem = ROUTE_MMA_ROWS * (zstride + ROUTE_WARPS * np) * sizeof(float);
+    const int outs = E + (has_gate ? 1 : 0), np = outs <= 32 ? 32 : outs <= 40 ? 40 : 64, mp = outs <= 32 ? 32 : 64;
+    const size_t mma_smem = ROUTE_MMA_ROWS * (zstride + ROUTE_WARPS * mp) * sizeof(float);
     if (!w_f32 && (D % 8) == 0 && (ldh % 8) == 0 && ((reinterpret_cast<uintptr_t>(h) | reinterpret_cast<uintptr_t>(wr)) & 15) == 0 &&
         mma_smem <= 200 * 1024) {
       const dim3 grid((rows + ROUTE_MMA_ROWS - 1) / ROUTE_MMA_ROWS);
@@ -708,9 +708,13 @@ int launch_moe_route(const void* h, int ldh, const void* wr, int w_f32, int rows
         return pdl_launch_cluster(few, dim3(grid.x * ROUTE_WARPS), dim3(np * 4), few_smem, s, ROUTE_WARPS, (const bf16*)h, ldh,
                                   (const bf16*)wr, rows, D, weights_ready, choice);
       }
-      auto kernel = np == 32 ? moe_route_mma_kernel<4> : np == 40 ? moe_route_mma_kernel<5> : moe_route_mma_kernel<8>;
+      // Launched the ordinary way: these few blocks, started early, gather on the SMs that the kernel before leaves first (norm
+      // and router of 1,024 rows of 2,048: 22.4 us early, 18.7 so).  A five-tile form for 33 to 40 outputs is slower than the one of
+      // eight (33 outputs, 2,048 rows, cold: 34.8 against 30 us).
+      auto kernel = mp == 32 ? moe_route_mma_kernel<4> : moe_route_mma_kernel<8>;
       if (mma_smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mma_smem);
-      return pdl_launch(kernel, grid, dim3(ROUTE_WARPS * 32), mma_smem, s, (const bf16*)h, ldh, (const bf16*)wr, rows, D, choice);
+      kernel<<<grid, ROUTE_WARPS * 32, mma_smem, s>>>((const bf16*)h, ldh, (const bf16*)wr, rows, D, choice);
+      return KVCM_LAUNCH_RESULT();
     }
   }
   const int vec = w_f32 ? 4 : RouteVec<T>::N;
