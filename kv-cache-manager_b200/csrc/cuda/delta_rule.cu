@@ -547,14 +547,14 @@ int launch_delta_conv(const void* proj, int ldp, const float* conv_w, int taps, 
                       state_stride, conv_off, seq_q_start, seq_state_slot, out, channels, bias);
   }
   if (taps <= kConvMaxTaps)
-    pdl_launch(delta_conv_run_kernel<T>, dim3((rows + kConvRun - 1) / kConvRun, by), dim3(256), 0, s, (const T*)proj, ldp, conv_w,
+    pdl_launch_if(false, delta_conv_run_kernel<T>, dim3((rows + kConvRun - 1) / kConvRun, by), dim3(256), 0, s, (const T*)proj, ldp, conv_w,
                taps, state, state_stride, conv_off, row_seq, seq_q_start, seq_state_slot, out, channels, rows, bias);
   else
-    pdl_launch(delta_conv_kernel<T>, dim3(rows, by), dim3(256), 0, s, (const T*)proj, ldp, conv_w, taps, state, state_stride,
+    pdl_launch_if(false, delta_conv_kernel<T>, dim3(rows, by), dim3(256), 0, s, (const T*)proj, ldp, conv_w, taps, state, state_stride,
                conv_off, row_seq, seq_q_start, seq_state_slot, out, channels, bias);
   int rc = KVCM_LAUNCH_RESULT();
   if (rc || taps == 1) return rc;
-  return pdl_launch(delta_conv_state_kernel<T>, dim3(seqs, by), dim3(256), 0, s, (const T*)proj, ldp, taps, state, state_stride,
+  return pdl_launch_if(false, delta_conv_state_kernel<T>, dim3(seqs, by), dim3(256), 0, s, (const T*)proj, ldp, taps, state, state_stride,
                     conv_off, seq_q_start, seq_q_len, seq_state_slot, channels);
 }
 
@@ -590,7 +590,9 @@ KVCM_API int kvcm_delta_scan_max_dk() { return 256; }
 
 // `rows`: rows of the step.  When every request brings one row (rows == seqs) the kernel is bound by
 // reading and writing the state: four lanes a column then, so that a warp's access covers whole
-// 32-byte sectors of a row of S.
+// 32-byte sectors of a row of S.  Portions are launched the ordinary way: a block's chain is long, and started early two
+// of them gather on an SM while another has none (convolution, preparation, scan and gated norm of one request of 300 rows, 16
+// heads of 128: 140.7 us early, 89.5 so; 512 rows 142; four requests of 2,048 rows in all 262 either way).
 template <int MODE>
 static int launch_scan(const ScanArgs& A, int rows, int seqs, cudaStream_t s) {
   const int heads = A.heads, dk = A.dk, dv = A.dv;
@@ -613,7 +615,7 @@ static int launch_scan(const ScanArgs& A, int rows, int seqs, cudaStream_t s) {
   // with a decay per channel a third staged array shares the static shared memory: fewer tokens a tile
   constexpr int TT_LONG = CHD ? 8 : 16, TT_LONGEST = CHD ? 4 : 8;
 #define KVCM_SCAN_E(COLS, LANES, NI, TT, EARLY)                                                                     \
-  pdl_launch((delta_scan_kernel<COLS, LANES, NI, TT, EARLY, MODE>), dim3((dv + COLS - 1) / COLS, heads, seqs),      \
+  pdl_launch_if(single_rows, delta_scan_kernel<COLS, LANES, NI, TT, EARLY, MODE>, dim3((dv + COLS - 1) / COLS, heads, seqs), \
              dim3(COLS * LANES), 0, s, A)
 #define KVCM_SCAN_C(COLS, LANES, NI, TT)                                                                            \
   do {                                                                                                              \

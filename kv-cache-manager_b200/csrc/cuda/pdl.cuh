@@ -26,8 +26,10 @@ __device__ __forceinline__ void pdl_wait() {
   asm volatile("griddepcontrol.wait;\n" ::: "memory");
 }
 
+// `early` false: the ordinary launch.  Blocks that start early gather on the SMs that the kernel before leaves first and stay
+// there, so a grid of few blocks that then work for long, or that are bound by what one SM can ask for, is better off with it.
 template <typename Kernel, typename... Args>
-int pdl_launch(Kernel kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+int pdl_launch_if(bool early, Kernel kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -37,8 +39,12 @@ int pdl_launch(Kernel kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t s
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = early ? 1 : 0;
   return static_cast<int>(cudaLaunchKernelEx(&cfg, kernel, args...));
+}
+template <typename Kernel, typename... Args>
+int pdl_launch(Kernel kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+  return pdl_launch_if(true, kernel, grid, block, smem, stream, args...);
 }
 
 // The same with the grid cut into thread-block clusters of `cluster_x` blocks along x (which must
