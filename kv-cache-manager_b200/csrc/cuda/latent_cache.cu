@@ -95,21 +95,44 @@ latent_q_rope_kernel(const float* q, int ldq, const int* __restrict__ positions,
   pdl_wait();
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  for (int h = warp; h < H; h += nwarps) {
-    const float* src = q + size_t(row) * ldq + size_t(h) * (dn + dr);
-    T* qn = qn_out + (size_t(row) * H + h) * dn;
-    for (int i = lane; i < dn; i += 32) stf(qn + i, src[i]);
-    T* dst = qrow + (size_t(row) * H + h) * HD + R;
-    const float* r = src + dn;
-    for (int j = lane; j < half; j += 32) {
-      const int ia = interleaved ? 2 * j : j, ib = interleaved ? 2 * j + 1 : j + half;
-      float a, b;
-      rotate_pair(r[ia], r[ib], cs_table[j], cs_table[half + j], a, b);
-      stf(dst + ia, a);
-      stf(dst + ib, b);
+  // Up to HEADS heads of a warp at a time: a lane's first KEEP unrotated elements and its first pair of each are asked for
+  // before the first store.
+  constexpr int HEADS = 4, KEEP = 4;
+  for (int h0 = warp; h0 < H; h0 += HEADS * nwarps) {
+    float v[HEADS][KEEP], x[HEADS], y[HEADS];
+    const int ia0 = interleaved ? 2 * lane : lane, ib0 = interleaved ? 2 * lane + 1 : lane + half;
+#pragma unroll
+    for (int u = 0; u < HEADS; ++u) {
+      const int h = h0 + u * nwarps;
+      if (h >= H) break;
+      const float* src = q + size_t(row) * ldq + size_t(h) * (dn + dr);
+#pragma unroll
+      for (int k = 0; k < KEEP; ++k) v[u][k] = lane + 32 * k < dn ? src[lane + 32 * k] : 0.f;
+      x[u] = lane < half ? src[dn + ia0] : 0.f;
+      y[u] = lane < half ? src[dn + ib0] : 0.f;
     }
-    for (int i = rot + lane; i < dr; i += 32) stf(dst + i, r[i]);
-    for (int i = dr + lane; i < HD - R; i += 32) stf(dst + i, 0.f);
+#pragma unroll
+    for (int u = 0; u < HEADS; ++u) {
+      const int h = h0 + u * nwarps;
+      if (h >= H) break;
+      const float* src = q + size_t(row) * ldq + size_t(h) * (dn + dr);
+      T* qn = qn_out + (size_t(row) * H + h) * dn;
+#pragma unroll
+      for (int k = 0; k < KEEP; ++k)
+        if (lane + 32 * k < dn) stf(qn + lane + 32 * k, v[u][k]);
+      for (int i = lane + 32 * KEEP; i < dn; i += 32) stf(qn + i, src[i]);
+      T* dst = qrow + (size_t(row) * H + h) * HD + R;
+      const float* r = src + dn;
+      for (int j = lane; j < half; j += 32) {
+        const int ia = interleaved ? 2 * j : j, ib = interleaved ? 2 * j + 1 : j + half;
+        float a, b;
+        rotate_pair(j == lane ? x[u] : r[ia], j == lane ? y[u] : r[ib], cs_table[j], cs_table[half + j], a, b);
+        stf(dst + ia, a);
+        stf(dst + ib, b);
+      }
+      for (int i = rot + lane; i < dr; i += 32) stf(dst + i, r[i]);
+      for (int i = dr + lane; i < HD - R; i += 32) stf(dst + i, 0.f);
+    }
   }
 }
 

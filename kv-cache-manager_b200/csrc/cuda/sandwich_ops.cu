@@ -353,9 +353,19 @@ concat_cast_kernel(const float* a, const float* b, T* __restrict__ out, int H) {
   pdl_launch_dependents();
   pdl_wait();
   const size_t t = blockIdx.x;
-  for (int i = threadIdx.x; i < H; i += blockDim.x) {
-    stf(out + t * 2 * H + i, a[t * H + i]);
-    stf(out + t * 2 * H + H + i, b[t * H + i]);
+  constexpr int AHEAD = 4;                           // elements of either row asked for before the first store
+  for (int i0 = threadIdx.x; i0 < H; i0 += AHEAD * blockDim.x) {
+    float va[AHEAD], vb[AHEAD];
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u) {
+      const int i = i0 + u * blockDim.x;
+      if (i < H) { va[u] = a[t * H + i]; vb[u] = b[t * H + i]; }
+    }
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u) {
+      const int i = i0 + u * blockDim.x;
+      if (i < H) { stf(out + t * 2 * H + i, va[u]); stf(out + t * 2 * H + H + i, vb[u]); }
+    }
   }
 }
 
