@@ -90,10 +90,22 @@ constexpr int kRopeTableMinRows = 64;                   // from here on the angl
 // without: 1 row 881 -> 809 us, 4 rows 902 -> 837, 8 rows 916 -> 869, 16 rows 1171 -> 1180).
 constexpr int kNormRideMaxRows = 8;
 // Rows of a step whose products run split over K on the tensor cores, norms, rotary encoding and activation in their
-// ends (gemm_tcgen05_splitk.cu).  The products of a layer of the 1.1B shape in us, against the library's (up to 16 rows the
-// streaming kernel's) with the separate kernels: 16 rows 31 against 36, 32 rows 35 against 43, 64 rows 42 against 45, 128 rows
-// 56 against 45.
+// ends (gemm_tcgen05_splitk.cu): 9 to 64 rows; up to 16 of them only where the streaming kernel does not take every product
+// of a layer.  Narrow models split K too little to keep the device busy, so that the ends of many rows queue in a few blocks:
+// a hidden size of 768 from 17 rows on, 1,024 from 33 on.  Whole decode steps in us at contexts of about 150, split against the
+// library (up to 16 rows the streaming kernel) with the separate kernels:
+//   16 rows : hidden 768 397 | 314, 1,024 536 | 417, 1,536 689 | 624, 2,048 (22 layers) 892 | 860; 3,072 (28 MB and more a
+//             product) 1,206 | 1,395, the 7B shape 3,490 | 4,430, the 8B shape 3,250 | 4,140
+//   32 rows : 96 (three layers) 105 | 72, 768 424 | 455, 1,024 546 | 640, 1,536 720 | 890, 2,048 938 | 1,158
+//   64 rows : 96 138 | 78, 768 547 | 512, 1,024 616 | 622, 1,536 810 | 908, 2,048 1,073 | 1,186, 3,072 1,540 | 1,650
 constexpr int kSplitkMinRows = 9, kSplitkMaxRows = 64;
+inline int splitk_min_hidden(int rows) { return rows <= 32 ? 768 : 1024; }
+// A product by itself of up to 64 rows that the streaming kernel does not take: split over K from 5 MB of weights on and up to
+// 65,536 outputs.  In us, split | library: 24 rows of [2048, 256] 3.7 | 2.6, [1024, 1024] 4.6 | 4.2, [4096, 512] 4.7 | 3.8, [1024, 2816]
+// 5.3 | 6.9, [32000, 2048] 23.1 | 24.9, [128256, 2048] 87.9 | 81.2, [128256, 4096] 164.8 | 163.1 (64 rows 177 | 188); 1 to 8 rows of
+// [4096, 11008] 17.8 | 26, [4096, 14336] 21.7 | 23.
+constexpr long long kSplitkMinBytes = 5ll << 20;
+constexpr int kSplitkMaxOutputs = 1 << 16;
 
 }  // namespace
 
@@ -137,7 +149,7 @@ int product(const KvcmForwardArgs& a, const void* x, const void* w, void* y, int
   if (a.f32) return kvcm_gemm_f32(x, w, y, M, N, K, K, K, N, 1, s);
   if ((M <= 8 || (long long)N * K * 2 <= kStreamMaxBytes) && kvcm_gemm_stream_supports(M, N, K))
     return kvcm_gemm_stream_bf16(x, w, y, M, N, K, K, K, N, out_f32 ? 1 : 0, a.sm_count, s);
-  if (M <= kSplitkMaxRows && kvcm_gemm_tcgen05_splitk_supports(M, N, K, K, K) &&
+  if (M <= kSplitkMaxRows && (long long)N * K * 2 >= kSplitkMinBytes && N <= kSplitkMaxOutputs && kvcm_gemm_tcgen05_splitk_supports(M, N, K, K, K) &&
       ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) == 0)
     return kvcm_gemm_tcgen05_splitk_bf16(x, w, y, M, N, K, K, K, N, out_f32 ? 1 : 0, 1, s);
   return library_gemm(a, x, w, y, M, N, K, out_f32, s);
@@ -241,13 +253,21 @@ KVCM_API int kvcm_forward(const KvcmForwardArgs* ap, int* launches, void* stream
   };
   const bool may_ride = !a.f32 && a.norm_partials != nullptr && a.norm_partials_floats >= (long long)ss_tiles * 16 &&
                         T <= kNormRideMaxRows;
+  const bool gate_fused = !a.f32 && (I % 8) == 0 && kvcm_gemm_stream_fused_supports(T, 2 * I, H);
+  const auto qkv_fused = [&](const KvcmForwardLayer& L) {
+    return !a.f32 && L.writes && (a.hd % 16) == 0 && kvcm_gemm_stream_fused_supports(T, QKV, H);
+  };
   // A few dozen rows: the same on the tensor cores, every product of the step or none.
   const auto aligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
   bool split = !a.f32 && a.norm_partials != nullptr && a.norm_partials_floats >= kvcm_splitk_norm_floats(H) &&
-               T >= kSplitkMinRows && T <= kSplitkMaxRows && a.rope_table != nullptr && a.rope_table_floats >= (long long)T * a.hd &&
+               T >= kSplitkMinRows && T <= kSplitkMaxRows && H >= splitk_min_hidden(T) && a.rope_table != nullptr &&
+               a.rope_table_floats >= (long long)T * a.hd &&
                (a.hd == 16 || a.hd == 32 || a.hd == 64 || a.hd == 128) && (H % 8) == 0 && (I % 8) == 0 && (QK % 8) == 0 &&
                kvcm_splitk_fused_supports(T, H, QK) && kvcm_splitk_fused_supports(T, H, I) && kvcm_splitk_fused_supports(T, I, H) &&
                aligned(a.x) && aligned(a.h) && aligned(a.qkv) && aligned(a.attn) && aligned(a.act) && aligned(a.rope_table);
+  bool all_stream = T <= 16 && gate_fused && streams(H, QK) && streams(H, I);
+  for (int l = 0; l < a.num_layers; ++l) all_stream = all_stream && qkv_fused(a.layers[l]);
+  split = split && !all_stream;
   for (int l = 0; l < a.num_layers; ++l) {
     const KvcmForwardLayer& L = a.layers[l];
     split = split && L.writes && aligned(L.w_qkv) && aligned(L.w_o) && aligned(L.w_gate_up) && aligned(L.w_down) &&
@@ -257,10 +277,6 @@ KVCM_API int kvcm_forward(const KvcmForwardArgs* ap, int* launches, void* stream
   // (each sublayer by itself: where the down product is too wide for the streaming kernel, as at the
   // Llama-3-8B shape, the attention sublayer still closes this way)
   const bool ride_attn = may_ride && streams(H, QK), ride_ffn = may_ride && streams(H, I);
-  const bool gate_fused = !a.f32 && (I % 8) == 0 && kvcm_gemm_stream_fused_supports(T, 2 * I, H);
-  const auto qkv_fused = [&](const KvcmForwardLayer& L) {
-    return !a.f32 && L.writes && (a.hd % 16) == 0 && kvcm_gemm_stream_fused_supports(T, QKV, H);
-  };
 
   KVCM_TRY(embed(a.tokens, a.embed, a.x, T, H, a.V, s)); ++n;
   bool table_filled = false;                            // the step's cosines and sines are in a.rope_table

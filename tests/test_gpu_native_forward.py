@@ -106,3 +106,29 @@ def test_host_time_of_a_prefill_step(model_folders):
             best = min(best, t1 - t0)
         host[native] = best
     assert host[True] < 0.8 * host[False], host
+
+
+@pytest.mark.parametrize("hidden,rows,form", [(768, 9, "stream"), (768, 16, "stream"), (768, 17, "split"), (768, 32, "split"), (768, 33, "library"),
+                                              (1024, 16, "stream"), (1024, 33, "split"), (1024, 64, "split"), (96, 17, "library")])
+def test_which_products_a_step_of_a_few_dozen_rows_takes(hidden, rows, form, tmp_path):
+    """Told by the launches: five a layer with the norms, rotary encoding and activation in the split-K products' ends, seven
+    with the streaming products, nine with the library's.  Logits against the plain implementation."""
+    import kvcm
+    from kvcm.kernels import library as K
+    dim, layers = (32, 3) if hidden < 128 else (64, 2)
+    heads = hidden // dim
+    cfg = kvcm.LlamaConfig(architecture="LlamaForCausalLM", vocab_size=500, hidden_size=hidden, intermediate_size=hidden * 2,
+                           num_hidden_layers=layers, num_attention_heads=heads, num_key_value_heads=heads // 3 if heads % 3 == 0 else heads // 4,
+                           head_dim=dim, max_position_embeddings=64, rope_theta=10000.0, rms_norm_eps=1e-5)
+    folder = str(tmp_path / "m")
+    kvcm.write_random_model(folder, cfg, seed=rows, dtype=torch.bfloat16)
+    r = helpers.Replayer(folder, "bfloat16", 16 * rows, 16, max_live=rows)
+    assert r.runner.native is not None
+    tokens = [(7 * i + 3) % 500 for i in range(rows)]
+    before = K.launch_count()
+    got = r.step([dict(id=f"r{i}", tokens=[t], want=[0]) for i, t in enumerate(tokens)])
+    # (embedding, final norm and head; with the split-K products the angles' table and the first norm)
+    assert K.launch_count() - before == {"stream": 3 + 7 * layers, "split": 5 + 5 * layers, "library": 3 + 9 * layers}[form]
+    c, w = P.read_model_folder(folder)
+    ref = torch.cat([P.llama_forward(c, w, [t], torch.bfloat16) for t in tokens])
+    helpers.assert_logits_close(got, ref, "bfloat16", form)
