@@ -20,7 +20,7 @@ BatchBuilder::BatchBuilder(int block_size, int max_blocks_per_seq, int num_group
 
 int64_t BatchBuilder::capacity_for(int rows, int seqs, int logit_rows) const {
   const int64_t tiles = rows / tile_rows_ + seqs + 1;
-  return round4(rows) * (4 + groups_) + round4(seqs) * 4 + round4(logit_rows) + round4(tiles) * 2 +
+  return round4(rows) * (4 + groups_) + round4(seqs) * 5 + round4(logit_rows) + round4(tiles) * 2 +
          round4(int64_t(groups_) * seqs * max_blocks_) + 64;
 }
 
@@ -87,6 +87,7 @@ BatchLayout BatchBuilder::build(const std::vector<BatchEntry>& entries, int32_t*
   L.off_tile_q0 = take(tiles);
   L.off_block_tables = take(int64_t(groups_) * L.seqs * max_blocks_);
   L.off_prev_tokens = take(L.rows);
+  L.off_decode_order = take(L.seqs);
   L.total_ints = at;
   if (at > capacity)
     throw std::runtime_error("batch: step needs " + std::to_string(at) + " ints, buffer holds " +
@@ -147,6 +148,12 @@ BatchLayout BatchBuilder::build(const std::vector<BatchEntry>& entries, int32_t*
     out[L.off_row_seq + row] = si;
     out[L.off_positions + row] = -1;          // context = position + 1 = 0 keys
   }
+  // Decode attention runs in several waves of blocks where requests and heads are many: a long context that starts last would
+  // run alone at the end.
+  int32_t* order = out + L.off_decode_order;
+  const int32_t* ctx = out + L.off_seq_ctx_len;
+  std::iota(order, order + L.seqs, 0);
+  std::stable_sort(order, order + L.decode_seqs + (L.seqs - L.real_seqs), [&](int32_t a, int32_t b) { return ctx[a] > ctx[b]; });
   int lr = 0;
   for (int e = 0; e < n_entries; ++e)
     for (int w : entries[e].want) out[L.off_logit_rows + lr++] = q_start_of[e] + w;

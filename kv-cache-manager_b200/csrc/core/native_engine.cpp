@@ -126,6 +126,7 @@ void NativeEngine::fill_args(KvcmForwardArgs& a, const BatchLayout& L, const int
   a.seq_q_start = base + L.off_seq_q_start;
   a.seq_q_len = base + L.off_seq_q_len;
   a.seq_ctx_len = base + L.off_seq_ctx_len;
+  a.decode_order = base + L.off_decode_order;
   a.tile_seq = base + L.off_tile_seq;
   a.tile_q0 = base + L.off_tile_q0;
   a.logit_rows = base + L.off_logit_rows;

@@ -40,7 +40,7 @@ struct DecodeParams {
   const float* sink;                   // per head, or null: exp(sink) joins the denominator where the result is normalised
   int log2_block;                      // log2(block_size) when it is a power of two, else -1
   int cluster_merge;                   // the partitions of a (request, head group) are one cluster
-  int by_length;                       // requests are taken longest first (at most kAttnThreads of them)
+  const int* order;                    // the order in which the requests are taken, or null: as they lie
 };
 
 constexpr int kTabMax = 512;         // page-table entries of a partition kept in shared memory
@@ -142,22 +142,7 @@ attn_decode_kernel(DecodeParams p) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, t4 = lane & 3;
 
-  // More blocks than run at once: the longest requests first, so that no long one starts when the rest is done.  Every
-  // block finds the blockIdx.z-th longest by itself (the lengths are inputs of the step, and few).  24 requests of 60 to 1,524
-  // keys, 32 heads of 128: 45 us in the order of the batch, 34 in this one; 24 of 400 each: 31.
-  int seq = blockIdx.z;
-  if (p.by_length) {
-    const int n = gridDim.z, mine = tid < n ? p.seq_ctx_len[tid] : 0;
-    stab[tid] = mine;
-    __syncthreads();
-    int before = 0;
-    for (int j = 0; j < n; ++j) before += stab[j] > mine || (stab[j] == mine && j < tid);
-    __syncthreads();
-    if (tid < n && before == int(blockIdx.z)) stab[0] = tid;
-    __syncthreads();
-    seq = stab[0];
-    __syncthreads();
-  }
+  const int seq = p.order ? p.order[blockIdx.z] : blockIdx.z;
   const int ctx = p.seq_ctx_len[seq];
   const int lo = ctx > 0 ? first_visible(ctx - 1, p.window, p.chunk) : 0;
   const int pbeg = (p.chunk > 0 || p.window > 0 ? lo / kKeyTile * kKeyTile : 0) + part * p.part_size;
@@ -437,7 +422,7 @@ int decode_resident_blocks(int sm_count) {
 // instead of per two) and the fewer, larger blocks still all fit; two for a grid too large for
 // three (more blocks fit an SM: a second wave of blocks costs more than the shallower pipeline).
 template <int HD>
-int launch_decode(const DecodeParams& p, int seqs, int sm_count, cudaStream_t s) {
+int launch_decode(const DecodeParams& p, const int* order, int seqs, int sm_count, cudaStream_t s) {
   const int G = p.nh / p.nkv;
   const long long blocks = (long long)p.num_parts * p.nkv * ((G + 15) / 16) * seqs;
   if constexpr (HD <= 128) {                                       // (five stages of larger heads do not fit an SM)
@@ -445,8 +430,13 @@ int launch_decode(const DecodeParams& p, int seqs, int sm_count, cudaStream_t s)
       return launch_decode_staged<HD, 5>(p, seqs, s);
   }
   if (blocks > decode_resident_blocks<HD, 3>(sm_count)) {
+    // ... and between 1.3 and 6 waves of blocks the caller's order of the requests: longest first, so that no long one starts
+    // when the rest is done.  In us, as they lie | longest first: 32 KV heads of 128, 24 requests (1.7 waves) of 400 keys at the
+    // median 42 | 36, of 400 each 31 | 31; 64 requests (4.6) 98 | 87; 32 of 64, 64 requests (2.8) 54 | 45.  Fewer waves: 12 heads of
+    // 64, 64 requests (1.04) 29 | 31, 16 heads of 128, 24 requests (0.9) 29 | 30; more: 40 heads of 128, 100 requests (9) 117 | 128.
     DecodeParams q = p;
-    q.by_length = seqs > 1 && seqs <= kAttnThreads;
+    const long long at_once = decode_resident_blocks<HD, 2>(sm_count);
+    if (blocks * 10 >= 13 * at_once && blocks <= 6 * at_once) q.order = order;
     return launch_decode_staged<HD, 2>(q, seqs, s);
   }
   return launch_decode_staged<HD, 3>(p, seqs, s);
@@ -489,11 +479,12 @@ KVCM_API int kvcm_attention_decode_cluster_parts(void) { return kMaxClusterParts
 // `softcap` > 0: scaled scores are capped as cap * tanh(score / cap); `sink` (per head, optional): exp(sink)
 // joins the softmax's denominator.
 // `keep_first` > 0 (with a window): the first keep_first keys of every request stay visible.  `chunk` > 0: a row sees
-// only its own chunk of positions.  With a window or a chunk the num_parts partitions of part_size keys cover [its first key
+// only its own chunk of positions.  `order` (optional): a permutation of the requests, the order in which they are taken where
+// the blocks do not all run at once.  With a window or a chunk the num_parts partitions of part_size keys cover [its first key
 // rounded down to a tile of 64, context).
 KVCM_API int kvcm_attention_decode_keep_bf16(const void* q, int q_stride, void* out, int out_stride,
                                              const void* k_cache, const void* v_cache, const int* block_tables,
-                                             int max_blocks, const int* seq_ctx_len, int seqs, int nh, int nkv,
+                                             int max_blocks, const int* seq_ctx_len, const int* order, int seqs, int nh, int nkv,
                                              int hd, int block_size, float scale, int window, int keep_first, int chunk, int part_size,
                                              int num_parts, float* scratch, int cluster_merge, float softcap,
                                              const float* sink, void* stream) {
@@ -521,11 +512,11 @@ KVCM_API int kvcm_attention_decode_keep_bf16(const void* q, int q_stride, void* 
   p.scale_log2 = (softcap > 0.f ? softcap : scale) * 1.4426950408889634f;
   p.cap_pre = softcap > 0.f ? scale / softcap : 0.f;
   p.sink = sink;
-  p.by_length = 0;
+  p.order = nullptr;
   p.log2_block = -1;
   for (int b = 0; b < 16; ++b) if ((1 << b) == block_size) p.log2_block = b;
   int rc = KVCM_ERR_UNSUPPORTED;
-#define X(N) if (hd == N) rc = launch_decode<N>(p, seqs, sm_count, (cudaStream_t)stream);
+#define X(N) if (hd == N) rc = launch_decode<N>(p, order, seqs, sm_count, (cudaStream_t)stream);
   KVCM_FOR_HEAD_DIMS(X)
 #undef X
   if (rc != 0 || num_parts == 1 || cluster_merge) return rc;
@@ -540,7 +531,7 @@ KVCM_API int kvcm_attention_decode_capped_bf16(const void* q, int q_stride, void
                                                int num_parts, float* scratch, int cluster_merge, float softcap,
                                                const float* sink, void* stream) {
   return kvcm_attention_decode_keep_bf16(q, q_stride, out, out_stride, k_cache, v_cache, block_tables, max_blocks, seq_ctx_len,
-                                         seqs, nh, nkv, hd, block_size, scale, window, 0, 0, part_size, num_parts, scratch,
+                                         nullptr, seqs, nh, nkv, hd, block_size, scale, window, 0, 0, part_size, num_parts, scratch,
                                          cluster_merge, softcap, sink, stream);
 }
 

@@ -42,8 +42,8 @@ int kvcm_attention_plain_bf16(const void*, int, void*, int, const void*, const v
 int kvcm_attention_fast_supports(int);
 int kvcm_attention_decode_resident_blocks(int);
 int kvcm_attention_decode_cluster_parts(void);
-int kvcm_attention_decode_bf16(const void*, int, void*, int, const void*, const void*, const int*, int, const int*, int, int,
-                               int, int, int, float, int, int, int, float*, int, void*);
+int kvcm_attention_decode_keep_bf16(const void*, int, void*, int, const void*, const void*, const int*, int, const int*, const int*, int,
+                                    int, int, int, int, float, int, int, int, int, int, float*, int, float, const float*, void*);
 int kvcm_attention_tcgen05_supports(int, int);
 int kvcm_attention_prefill_tcgen05_bf16(const void*, int, int, void*, int, const void*, const void*, int, const int*, int,
                                         const int*, const int*, const int*, const int*, const int*, int, int, int, int, int,
@@ -90,20 +90,21 @@ constexpr int kRopeTableMinRows = 64;                   // from here on the angl
 // without: 1 row 881 -> 809 us, 4 rows 902 -> 837, 8 rows 916 -> 869, 16 rows 1171 -> 1180).
 constexpr int kNormRideMaxRows = 8;
 // Rows of a step whose products run split over K on the tensor cores, norms, rotary encoding and activation in their
-// ends (gemm_tcgen05_splitk.cu): 9 to 64 rows; up to 16 of them only where the streaming kernel does not take every product
-// of a layer.  Narrow models split K too little to keep the device busy, so that the ends of many rows queue in a few blocks:
-// a hidden size of 768 from 17 rows on, 1,024 from 33 on.  Whole decode steps in us at contexts of about 150, split against the
-// library (up to 16 rows the streaming kernel) with the separate kernels:
-//   16 rows : hidden 768 397 | 314, 1,024 536 | 417, 1,536 689 | 624, 2,048 (22 layers) 892 | 860; 3,072 (28 MB and more a
+// ends (gemm_tcgen05_splitk.cu): 9 to 64 rows, up to 16 of them only where the streaming kernel does not take every product
+// of a layer, of models of a hidden size of 1,536 and more.  Narrower ones split K too little to keep the device busy, so that
+// the ends of many rows queue in a few blocks.  Whole decode steps in us at contexts of 150, split against the library (up to 16
+// rows the streaming kernel) with the separate kernels, each in a process of its own:
+//   16 rows : hidden 768 397 | 314, 1,024 536 | 431, 1,536 689 | 624, 2,048 (22 layers) 892 | 860; 3,072 (28 MB and more a
 //             product) 1,206 | 1,395, the 7B shape 3,490 | 4,430, the 8B shape 3,250 | 4,140
-//   32 rows : 96 (three layers) 105 | 72, 768 424 | 455, 1,024 546 | 640, 1,536 720 | 890, 2,048 938 | 1,158
-//   64 rows : 96 138 | 78, 768 547 | 512, 1,024 616 | 622, 1,536 810 | 908, 2,048 1,073 | 1,186, 3,072 1,540 | 1,650
-constexpr int kSplitkMinRows = 9, kSplitkMaxRows = 64;
-inline int splitk_min_hidden(int rows) { return rows <= 32 ? 768 : 1024; }
-// A product by itself of up to 64 rows that the streaming kernel does not take: split over K from 5 MB of weights on and up to
-// 65,536 outputs.  In us, split | library: 24 rows of [2048, 256] 3.7 | 2.6, [1024, 1024] 4.6 | 4.2, [4096, 512] 4.7 | 3.8, [1024, 2816]
-// 5.3 | 6.9, [32000, 2048] 23.1 | 24.9, [128256, 2048] 87.9 | 81.2, [128256, 4096] 164.8 | 163.1 (64 rows 177 | 188); 1 to 8 rows of
-// [4096, 11008] 17.8 | 26, [4096, 14336] 21.7 | 23.
+//   24 rows : 96 (three layers) 105 | 72, 768 417 | 389, 1,024 555 | 547, 1,536 716 | 797, 2,048 925 | 1,045
+//   32 rows : 768 428 | 400, 1,024 548 | 557, 1,536 717 | 809, 2,048 941 | 1,059
+//   64 rows : 96 138 | 78, 768 548 | 454, 1,024 618 | 549, 1,536 806 | 826, 2,048 1,067 | 1,086
+constexpr int kSplitkMinRows = 9, kSplitkMaxRows = 64, kSplitkMinHidden = 1536;
+// A product by itself of up to 64 rows that the streaming kernel does not take: split over K from that K and 5 MB of weights on
+// and up to 65,536 outputs.  In us, split | library: 24 rows of [2048, 256] 3.7 | 2.6, [1024, 1024] 4.6 | 4.2, [4096, 512] 4.7 |
+// 3.8, [1024, 2816] 5.3 | 6.9, [32000, 2048] 23.1 | 24.9, [128256, 2048] 87.9 | 81.2, [128256, 4096] 164.8 | 163.1 (64 rows 177 |
+// 188); 1 to 8 rows of [4096, 11008] 17.8 | 26, [4096, 14336] 21.7 | 23.  A step of 64 rows at a hidden size of 768 with its
+// gate/up products split 474, without 455.
 constexpr long long kSplitkMinBytes = 5ll << 20;
 constexpr int kSplitkMaxOutputs = 1 << 16;
 
@@ -149,7 +150,8 @@ int product(const KvcmForwardArgs& a, const void* x, const void* w, void* y, int
   if (a.f32) return kvcm_gemm_f32(x, w, y, M, N, K, K, K, N, 1, s);
   if ((M <= 8 || (long long)N * K * 2 <= kStreamMaxBytes) && kvcm_gemm_stream_supports(M, N, K))
     return kvcm_gemm_stream_bf16(x, w, y, M, N, K, K, K, N, out_f32 ? 1 : 0, a.sm_count, s);
-  if (M <= kSplitkMaxRows && (long long)N * K * 2 >= kSplitkMinBytes && N <= kSplitkMaxOutputs && kvcm_gemm_tcgen05_splitk_supports(M, N, K, K, K) &&
+  if (M <= kSplitkMaxRows && K >= kSplitkMinHidden && (long long)N * K * 2 >= kSplitkMinBytes && N <= kSplitkMaxOutputs &&
+      kvcm_gemm_tcgen05_splitk_supports(M, N, K, K, K) &&
       ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) == 0)
     return kvcm_gemm_tcgen05_splitk_bf16(x, w, y, M, N, K, K, K, N, out_f32 ? 1 : 0, 1, s);
   return library_gemm(a, x, w, y, M, N, K, out_f32, s);
@@ -200,9 +202,9 @@ int attention(const KvcmForwardArgs& a, const KvcmForwardLayer& L, const void* q
     int in_cluster = parts > 1 && parts <= cluster;
     if (parts > 1 && !in_cluster && (long long)nd * a.nh * parts * (a.hd + 2) > a.attn_scratch_floats)
       return KVCM_ERR_UNSUPPORTED;                                  // the caller sizes the scratch for its limits
-    rc = kvcm_attention_decode_bf16(q, q_stride, a.attn, a.nh * a.hd, L.k_cache, L.v_cache, tables, a.max_blocks,
-                                    a.seq_ctx_len, nd, a.nh, a.nkv, a.hd, a.block_size, a.scale, L.window, size, parts,
-                                    a.attn_scratch, in_cluster, s);
+    rc = kvcm_attention_decode_keep_bf16(q, q_stride, a.attn, a.nh * a.hd, L.k_cache, L.v_cache, tables, a.max_blocks,
+                                         a.seq_ctx_len, a.decode_order, nd, a.nh, a.nkv, a.hd, a.block_size, a.scale, L.window, 0, 0,
+                                         size, parts, a.attn_scratch, in_cluster, 0.f, nullptr, s);
     if (rc) return rc;
     launches += (parts > 1 && !in_cluster) ? 2 : 1;
   }
@@ -260,7 +262,7 @@ KVCM_API int kvcm_forward(const KvcmForwardArgs* ap, int* launches, void* stream
   // A few dozen rows: the same on the tensor cores, every product of the step or none.
   const auto aligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
   bool split = !a.f32 && a.norm_partials != nullptr && a.norm_partials_floats >= kvcm_splitk_norm_floats(H) &&
-               T >= kSplitkMinRows && T <= kSplitkMaxRows && H >= splitk_min_hidden(T) && a.rope_table != nullptr &&
+               T >= kSplitkMinRows && T <= kSplitkMaxRows && H >= kSplitkMinHidden && a.rope_table != nullptr &&
                a.rope_table_floats >= (long long)T * a.hd &&
                (a.hd == 16 || a.hd == 32 || a.hd == 64 || a.hd == 128) && (H % 8) == 0 && (I % 8) == 0 && (QK % 8) == 0 &&
                kvcm_splitk_fused_supports(T, H, QK) && kvcm_splitk_fused_supports(T, H, I) && kvcm_splitk_fused_supports(T, I, H) &&

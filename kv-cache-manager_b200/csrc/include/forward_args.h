@@ -20,7 +20,7 @@ struct KvcmForwardArgs {
   const float* inv_freq;
   // the step: the batch's integer arrays on the device
   const int* tokens; const int* positions; const int* row_seq; const int* seq_q_start; const int* seq_q_len;
-  const int* seq_ctx_len; const int* tile_seq; const int* tile_q0; const int* logit_rows;
+  const int* seq_ctx_len; const int* decode_order; const int* tile_seq; const int* tile_q0; const int* logit_rows;
   const int* group_tables[KVCM_FORWARD_MAX_GROUPS]; const int* group_slots[KVCM_FORWARD_MAX_GROUPS];
   // buffers of the caller, sized for the step: x [T,H] float; h, proj [T,H]; qkv [T,QKV]; attn [T,nh*hd];
   // gate_up [T,2I]; act [T,I]; h_last [L,H]; logits [L,V] float; attn_scratch floats; a library workspace;

@@ -154,6 +154,7 @@ class NativeForward:
         a.tokens, a.positions, a.row_seq = ctx.tokens.data_ptr(), ctx.positions.data_ptr(), ctx.row_seq.data_ptr()
         a.seq_q_start, a.seq_q_len = ctx.seq_q_start.data_ptr(), ctx.seq_q_len.data_ptr()
         a.seq_ctx_len = ctx.seq_ctx_len.data_ptr()
+        a.decode_order = ctx.decode_order.data_ptr() if ctx.decode_order is not None else None
         a.tile_seq, a.tile_q0 = ctx.tile_seq.data_ptr(), ctx.tile_q0.data_ptr()
         a.logit_rows = ctx.logit_rows.data_ptr()
         for g, view in enumerate(ctx.groups):

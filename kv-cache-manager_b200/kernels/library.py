@@ -487,8 +487,13 @@ def attention_decode(q: torch.Tensor, out: torch.Tensor, k_cache: torch.Tensor, 
                      keep_first: int = 0, chunk: int = 0) -> None:
     """Single-row entries: q/out hold one row per request, in the order of the batch's entries.
     ``softcap`` / ``sink`` / ``chunk`` as in ``attention_plain``; with a window or
-    chunks the partitions split the longest part of a context that one can hold (and the tile its start lies in)."""
-    _cuda(q, out, k_cache, v_cache, block_tables, sink)
+    chunks the partitions split the longest part of a context that one can hold (and the tile its start lies in).
+    ``ctx.decode_order`` (optional, int32 [requests], a permutation): the order in which the requests are taken where the
+    blocks do not all run at once."""
+    order = getattr(ctx, "decode_order", None)
+    _cuda(q, out, k_cache, v_cache, block_tables, sink, order)
+    _need(order is None or (order.dtype == _I32 and order.is_contiguous() and order.numel() >= q.shape[0]),
+          "attention_decode: decode_order int32 [requests]")
     _need(sink is None or (sink.dtype == torch.float32 and sink.is_contiguous() and sink.numel() == nh),
           "attention_decode: sink float32 [heads]")
     S = q.shape[0]
@@ -510,7 +515,7 @@ def attention_decode(q: torch.Tensor, out: torch.Tensor, k_cache: torch.Tensor, 
         scratch = torch.empty(n, dtype=torch.float32, device=q.device)
     rc = _lib().kvcm_attention_decode_keep_bf16(
         _p(q), q.stride(0), _p(out), out.stride(0), _p(k_cache), _p(v_cache), _p(block_tables),
-        block_tables.shape[1], _p(ctx.seq_ctx_len), S, nh, nkv, hd, k_cache.shape[2],
+        block_tables.shape[1], _p(ctx.seq_ctx_len), _p(order), S, nh, nkv, hd, k_cache.shape[2],
         ctypes.c_float(scale), int(window), int(keep_first), int(chunk), size, parts, _p(scratch), int(in_cluster), ctypes.c_float(softcap), _p(sink),
         _stream())
     _check(rc, "attention_decode", f"(hd={hd}, nh={nh}, nkv={nkv})")
@@ -917,7 +922,7 @@ class ForwardArgs(ctypes.Structure):
         ("lm_head", ctypes.c_void_p), ("inv_freq", ctypes.c_void_p),
         ("tokens", ctypes.c_void_p), ("positions", ctypes.c_void_p), ("row_seq", ctypes.c_void_p),
         ("seq_q_start", ctypes.c_void_p), ("seq_q_len", ctypes.c_void_p), ("seq_ctx_len", ctypes.c_void_p),
-        ("tile_seq", ctypes.c_void_p), ("tile_q0", ctypes.c_void_p), ("logit_rows", ctypes.c_void_p),
+        ("decode_order", ctypes.c_void_p), ("tile_seq", ctypes.c_void_p), ("tile_q0", ctypes.c_void_p), ("logit_rows", ctypes.c_void_p),
         ("group_tables", ctypes.c_void_p * FORWARD_MAX_GROUPS), ("group_slots", ctypes.c_void_p * FORWARD_MAX_GROUPS),
         ("x", ctypes.c_void_p), ("h", ctypes.c_void_p), ("qkv", ctypes.c_void_p), ("attn", ctypes.c_void_p),
         ("proj", ctypes.c_void_p), ("gate_up", ctypes.c_void_p), ("act", ctypes.c_void_p), ("h_last", ctypes.c_void_p),

@@ -185,6 +185,7 @@ class StepContext:
     dtype: torch.dtype               # storage dtype of activations
     workspace: Any = None            # per-engine scratch provider (see engine.runner.Workspace)
     options: Dict[str, Any] = field(default_factory=dict)
+    decode_order: Optional[torch.Tensor] = None  # the single-row entries, longest context first
     prev_tokens: Optional[torch.Tensor] = None   # per row: the request's token one position earlier (-1 at position 0)
     h_stream: Optional[torch.Tensor] = None      # storage-dtype copy of the residual stream, kept current by blocks
                                                  # whose sublayers read the stream itself (None: nobody keeps one)

@@ -61,6 +61,16 @@ def test_padding_rows_read_and_write_nothing():
         build([(a, 0, 6, [])], pad_rows=8, pad_seqs=3)               # padding is for decode steps
 
 
+def test_single_rows_are_ordered_by_length_longest_first():
+    """Portions keep their places behind them, equal lengths their order; padding entries (no keys) come last."""
+    s = [seq_with_pages(i, range(20), [0, 1, 2, 3, 4]) for i in range(5)]
+    lay, buf = build([(s[0], 3, 1, []), (s[1], 0, 6, []), (s[2], 11, 1, []), (s[3], 3, 1, []), (s[4], 4, 2, [])])
+    assert lay.entry_order == [0, 2, 3, 1, 4] and arr(buf, lay.off_seq_ctx_len, 5) == [4, 12, 4, 6, 6]
+    assert arr(buf, lay.off_decode_order, 5) == [1, 0, 2, 3, 4]
+    lay, buf = build([(s[0], 3, 1, [0]), (s[1], 9, 1, [0])], pad_rows=4, pad_seqs=4, pad_logit_rows=4)
+    assert arr(buf, lay.off_decode_order, 4) == [1, 0, 2, 3]
+
+
 def test_layout_of_a_padded_shape_is_fixed():
     d1 = seq_with_pages(1, range(9), [1, 0, 4])
     d2 = seq_with_pages(2, range(3), [6])

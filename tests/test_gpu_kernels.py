@@ -839,8 +839,8 @@ def test_decode_attention_long_contexts_and_many_partitions():
 @pytest.mark.parametrize("hd,seqs", [(64, 40), (128, 24)])
 @pytest.mark.parametrize("lens", ["ragged", "equal"])
 def test_decode_attention_of_more_blocks_than_run_at_once(hd, seqs, lens):
-    """32 KV heads of `seqs` requests do not all run at once: the requests are then taken longest first, every block finding
-    its own.  Ragged lengths with ties and entries without a key, and equal lengths; undivided and in both merge forms."""
+    """32 KV heads of `seqs` requests do not all run at once: the requests are then taken in the caller's order.  Ragged lengths
+    with ties and entries without a key, and equal lengths; undivided and in both merge forms; longest first, and as they lie."""
     nh, g = 32, torch.Generator().manual_seed(seqs)
     assert nh * seqs > K()._decode_resident_blocks(hd, DEV)
     seq_lens = [130] * seqs
@@ -852,9 +852,14 @@ def test_decode_attention_of_more_blocks_than_run_at_once(hd, seqs, lens):
     ref = reference_attention(case, nh, nh, hd, hd ** -0.5, 0)
     for options in ({"attn_version": "v1"}, {"attn_parts": 3}, {"attn_parts": 3, "attn_merge": "kernel"}):
         case["ctx"].options = options
-        out = torch.full((seqs, nh * hd), float("nan"), dtype=torch.bfloat16, device=DEV)
-        K().attention_decode(case["q"], out, case["kc"], case["vc"], case["tables"], case["ctx"], nh, nh, hd, hd ** -0.5)
-        close(out, ref, "bfloat16", str(options))
+        bits = []
+        for order in (None, torch.tensor(seq_lens).argsort(descending=True, stable=True).to(torch.int32).to(DEV)):
+            case["ctx"].decode_order = order
+            out = torch.full((seqs, nh * hd), float("nan"), dtype=torch.bfloat16, device=DEV)
+            K().attention_decode(case["q"], out, case["kc"], case["vc"], case["tables"], case["ctx"], nh, nh, hd, hd ** -0.5)
+            close(out, ref, "bfloat16", str(options))
+            bits.append(out)
+        assert torch.equal(*bits)
 
 
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])

@@ -108,8 +108,8 @@ def test_host_time_of_a_prefill_step(model_folders):
     assert host[True] < 0.8 * host[False], host
 
 
-@pytest.mark.parametrize("hidden,rows,form", [(768, 9, "stream"), (768, 16, "stream"), (768, 17, "split"), (768, 32, "split"), (768, 33, "library"),
-                                              (1024, 16, "stream"), (1024, 33, "split"), (1024, 64, "split"), (96, 17, "library")])
+@pytest.mark.parametrize("hidden,rows,form", [(1536, 9, "stream"), (1536, 16, "stream"), (1536, 17, "split"), (1536, 64, "split"), (1024, 16, "stream"),
+                                              (1024, 17, "library"), (1024, 63, "library"), (96, 17, "library")])
 def test_which_products_a_step_of_a_few_dozen_rows_takes(hidden, rows, form, tmp_path):
     """Told by the launches: five a layer with the norms, rotary encoding and activation in the split-K products' ends, seven
     with the streaming products, nine with the library's.  Logits against the plain implementation."""

@@ -10,7 +10,7 @@ CUDA = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
 # Weights, and the integers of the batch and the keys and values of earlier tokens, which no kernel of a step writes.
 CONSTANTS = {"W", "wr", "wgu", "wd", "w", "weight", "wq", "wc", "wb", "wn", "w0", "w1", "mix", "outw", "inw", "lambda",
              "inv_freq", "v_inv_freq", "decay", "positions", "slot_mapping", "rows", "row_seq", "seq_q_start", "seq_q_len",
-             "seq_ctx_len", "seq_state_slot", "block_tables", "tile_seq", "tile_q0"}
+             "seq_ctx_len", "order", "seq_state_slot", "block_tables", "tile_seq", "tile_q0"}
 # Named above the wait: keys below the newest (written by earlier steps), and rows that a lambda copies behind it.
 BEHIND_IT = {"attn_decode_kernel": {"k_cache", "v_cache"}, "gemm_f32_kernel": {"X"}}
 
