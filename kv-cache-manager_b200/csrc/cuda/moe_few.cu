@@ -13,10 +13,9 @@
 // wait.)  A choice that names no expert is passed over and reported through the error word of the experts' products.
 // The k index inside a 32-wide block is permuted identically for both operands (thread t of a quad owns k = 8t..8t+7),
 // which makes every load a 16-byte vector.  Partial sums of the warps are added in warp order: reproducible.
-// Measured on B200 (32 experts of 512 x 2,048, a call alone with cold weights): 4 rows of 4 choices, 13 experts hit, 20 us; 8 rows of
-// 4, 22 experts, 34; 8 rows of 8, 30 experts, 40; 16 rows of 8, 43; the sorted form 48, 46, 53 and 53.  From 17 rows on they are
-// level.  Taken back: several tiles a block (gate/up 25 us in a step instead of 18), whole rows through shared memory by
-// asynchronous copies (26 instead of 20 us a call).
+// Measured on B200 (32 experts of 512 x 2,048, 8 choices a row, launches back to back): 1 row 16 us, 4 rows 35, 8 rows 43, 16
+// rows 50; the sorted form 30, 46, 50 and 50.  Several tiles a block and whole rows through shared memory by asynchronous copies
+// were both slower.
 #include "common.cuh"
 #include "pdl.cuh"
 

@@ -101,12 +101,12 @@ constexpr int kNormRideMaxRows = 8;
 //   64 rows : 96 138 | 78, 768 548 | 454, 1,024 618 | 549, 1,536 806 | 826, 2,048 1,067 | 1,086
 constexpr int kSplitkMinRows = 9, kSplitkMaxRows = 64, kSplitkMinHidden = 1536;
 // A product by itself of up to 64 rows that the streaming kernel does not take: split over K from that K and 5 MB of weights on
-// and up to 65,536 outputs.  In us, split | library: 24 rows of [2048, 256] 3.7 | 2.6, [1024, 1024] 4.6 | 4.2, [4096, 512] 4.7 |
+// and up to 65,536 outputs; beyond 32 rows of 8,192 outputs and more.  In us, split | library: 24 rows of [2048, 256] 3.7 | 2.6, [1024, 1024] 4.6 | 4.2, [4096, 512] 4.7 |
 // 3.8, [1024, 2816] 5.3 | 6.9, [32000, 2048] 23.1 | 24.9, [128256, 2048] 87.9 | 81.2, [128256, 4096] 164.8 | 163.1 (64 rows 177 |
 // 188); 1 to 8 rows of [4096, 11008] 17.8 | 26, [4096, 14336] 21.7 | 23.  A step of 64 rows at a hidden size of 768 with its
-// gate/up products split 474, without 455.
+// gate/up products split 474, without 455; at 1,024 with its down products split 568, without 549.
 constexpr long long kSplitkMinBytes = 5ll << 20;
-constexpr int kSplitkMaxOutputs = 1 << 16;
+constexpr int kSplitkMaxOutputs = 1 << 16, kSplitkWideOutputs = 1 << 13;
 
 }  // namespace
 
@@ -150,7 +150,8 @@ int product(const KvcmForwardArgs& a, const void* x, const void* w, void* y, int
   if (a.f32) return kvcm_gemm_f32(x, w, y, M, N, K, K, K, N, 1, s);
   if ((M <= 8 || (long long)N * K * 2 <= kStreamMaxBytes) && kvcm_gemm_stream_supports(M, N, K))
     return kvcm_gemm_stream_bf16(x, w, y, M, N, K, K, K, N, out_f32 ? 1 : 0, a.sm_count, s);
-  if (M <= kSplitkMaxRows && K >= kSplitkMinHidden && (long long)N * K * 2 >= kSplitkMinBytes && N <= kSplitkMaxOutputs &&
+  if (M <= (N >= kSplitkWideOutputs ? kSplitkMaxRows : 32) && K >= kSplitkMinHidden && (long long)N * K * 2 >= kSplitkMinBytes &&
+      N <= kSplitkMaxOutputs &&
       kvcm_gemm_tcgen05_splitk_supports(M, N, K, K, K) &&
       ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) == 0)
     return kvcm_gemm_tcgen05_splitk_bf16(x, w, y, M, N, K, K, K, N, out_f32 ? 1 : 0, 1, s);

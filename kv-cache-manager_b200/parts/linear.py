@@ -81,7 +81,7 @@ def matmul_nt(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype, options:
             K.gemm_tcgen05(x, w, y)
             return y
     # In between: the library, unless the caller wants this engine's kernels only (the split-K
-    # tcgen05 kernel: correct and reproducible, about half the library's speed at these sizes).
+    # tcgen05 kernel, which is the faster one for wide weights only: csrc/cuda/step_forward.cu has both sides' times).
     if (native or mode == "splitk") and K.splitk_gemm_supported(x, w):
         y = torch.empty((M, N), dtype=out_dtype, device=x.device)
         K.gemm_tcgen05_splitk(x, w, y, weights_ready=True)
